@@ -104,10 +104,15 @@ public:
     uint32_t* id[2] = {nullptr, nullptr};
     Real *density = nullptr, *factor = nullptr, *densityAdv = nullptr, *kcoef = nullptr;
     Vec4<Real>* acc = nullptr;
-    uint32_t *counts = nullptr, *nbr = nullptr;
+    uint32_t* counts = nullptr;
+    uint4* nbr = nullptr;
+    Vec4<Real>* coef = nullptr;
+    Real* vol = nullptr;
+    bool coef_ok = false;  // the pair coefficients match the lists and the current positions
     SortBuffers sb;
     uint2* ftab = nullptr;
     uint2* btab = nullptr;
+    uint8_t* bnear = nullptr;  // per cell: a boundary particle within two cells
     size_t cells = 0;
     Vec4<Real>* bpos[2] = {nullptr, nullptr};
     Vec4<Real>* bvel[2] = {nullptr, nullptr};
@@ -261,12 +266,12 @@ public:
         cap = s.neighbor_capacity;
         stride = (Nc + 31u) & ~31u;
         for (int b = 0; b < 2; ++b) {
-            DF_TRY(dalloc(&pos[b], Nc));
+            DF_TRY(dalloc(&pos[b], Nc + kScanPad));
             DF_TRY(dalloc(&vel[b], Nc));
             DF_TRY(dalloc(&kappa[b], Nc));
             DF_TRY(dalloc(&kappaV[b], Nc));
             DF_TRY(dalloc(&id[b], Nc));
-            DF_TRY(dalloc(&bpos[b], Bc));
+            DF_TRY(dalloc(&bpos[b], Bc + kScanPad));
             DF_TRY(dalloc(&bvel[b], Bc));
         }
         DF_TRY(dalloc(&density, Nc));
@@ -275,7 +280,9 @@ public:
         DF_TRY(dalloc(&kcoef, Nc));
         DF_TRY(dalloc(&acc, Nc));
         DF_TRY(dalloc(&counts, Nc));
-        DF_TRY(dalloc(&nbr, (size_t)cap * stride));
+        DF_TRY(dalloc(&nbr, (size_t)group_capacity(cap) * stride));
+        DF_TRY(dalloc(&coef, (size_t)group_capacity(cap) * stride));
+        DF_TRY(dalloc(&vol, Nc));
         DF_TRY(dalloc(&bid, Bc));
         DF_TRY(dalloc(&brest, (size_t)Bc * 3));
         const uint32_t nmax = std::max(Nc, Bc);
@@ -321,9 +328,9 @@ public:
         for (int b = 0; b < 2; ++b) {
             f(pos[b]); f(vel[b]); f(kappa[b]); f(kappaV[b]); f(id[b]); f(bpos[b]); f(bvel[b]);
         }
-        f(density); f(factor); f(densityAdv); f(kcoef); f(acc); f(counts); f(nbr); f(bid); f(bforce); f(bforce_fx);
+        f(density); f(factor); f(densityAdv); f(kcoef); f(acc); f(counts); f(nbr); f(coef); f(vol); f(bid); f(bforce); f(bforce_fx);
         f(sb.keys_a); f(sb.keys_b); f(sb.vals_a); f(sb.vals_b); f(sb.workspace);
-        f(partials); f(cfl_partials); f(ctl); f(status); f(stage); f(dl); f(ds); f(ftab); f(btab);
+        f(partials); f(cfl_partials); f(ctl); f(status); f(stage); f(dl); f(ds); f(ftab); f(btab); f(bnear);
         for (int b = 0; b < 2; ++b) {
             f(kappaT[b]); f(kappaVT[b]);
         }
@@ -422,6 +429,7 @@ public:
     }
 
     int sync_state() {
+        coef_ok = false;  // the particle order, the boundary or the lists may have changed
         hs.p = params();
         hs.pos = pos[cur];
         hs.vel = vel[cur];
@@ -435,6 +443,8 @@ public:
         hs.acc = acc;
         hs.counts = counts;
         hs.nbr = nbr;
+        hs.coef = coef;
+        hs.vol = vol;
         hs.bpos = bpos[0];
         hs.bvel = bvel[0];
         hs.partials = partials;
@@ -506,12 +516,16 @@ public:
         if (c != cells) {
             if (ftab) cudaFree(ftab);
             if (btab) cudaFree(btab);
+            if (bnear) cudaFree(bnear);
             ftab = btab = nullptr;
+            bnear = nullptr;
             DF_TRY(dalloc(&ftab, c));
             DF_TRY(dalloc(&btab, c));
+            DF_TRY(dalloc(&bnear, c));
             cells = c;
         }
         DF_CUDA(cudaMemsetAsync(btab, 0, cells * sizeof(uint2), stream));
+        DF_CUDA(cudaMemsetAsync(bnear, 0, cells, stream));
         grid_ready = true;
         return DFSPH_OK;
     }
@@ -550,7 +564,9 @@ public:
         launch_reorder_boundary<Real>(perm, nb, bpos[1], bvel[1], bpos[0], bvel[0], bid, stream);
         DF_CUDA(cudaMemsetAsync(btab, 0, cells * sizeof(uint2), stream));
         launch_cell_bounds(skeys, nb, dim[0], dim[1], dim[2], btab, stream);
-        launches += 3;
+        DF_CUDA(cudaMemsetAsync(bnear, 0, cells, stream));
+        launch_mark_near_boundary(skeys, nb, dim[0], dim[1], dim[2], bnear, stream);
+        launches += 4;
         if (compute_psi) {
             launch_boundary_psi<Real>(bpos[0], bpos[1], nb, p, btab, status, stream);
             DF_CUDA(cudaMemcpyAsync(bpos[0], bpos[1], (size_t)nb * sizeof(Vec4<Real>), cudaMemcpyDeviceToDevice,
@@ -742,6 +758,7 @@ public:
     int update_fluid(const float* xyz, const float* vxyz) {
         DF_CHECK(xyz, DFSPH_E_INVALID, "null fluid positions");
         if (!n) return DFSPH_OK;
+        coef_ok = false;
         float* sx = stage;
         float* sv = stage + (size_t)n * 3;
         DF_CUDA(cudaMemcpyAsync(sx, xyz, (size_t)n * 3 * sizeof(float), cudaMemcpyHostToDevice, stream));
@@ -791,7 +808,7 @@ public:
             DF_CUDA(cudaMemsetAsync(bforce_fx, 0, (size_t)nb * 3 * sizeof(unsigned long long), stream));
         if (!n) return DFSPH_OK;
         DF_TRY(bin_fluid(true));
-        launch_build_neighbors<Real>(ds, n, ftab, btab, stream, bshifted);
+        launch_build_neighbors<Real>(ds, n, ftab, btab, bnear, stream, bshifted);
         launches += 1;
         DF_TRY(flush_pending());  // velocities uploaded during the binning and the build
         if (corrupt_neighbor) {  // checked builds only (the key is rejected otherwise); one search
@@ -1245,7 +1262,7 @@ public:
             if (sc.enable_divergence_solver) {
                 DF_TRY(divergence_solve(sc.max_iterations_v, sc.max_error_v));
             } else {
-                launch_density_alpha<Real>(ds, n, false, false, stream);
+                density_pass(false, false);
                 launches += 1;
             }
             DF_TRY(external_forces(false));
@@ -1663,18 +1680,31 @@ public:
         return DFSPH_OK;
     }
 
+    // The density pass also writes the pair coefficients and m / rho, which the other passes read.
+    void density_pass(bool warm_v, bool features_out) {
+        launch_density_alpha<Real>(ds, n, warm_v, features_out, stream);
+        coef_ok = true;
+    }
+    // Both of these for a pass that no density pass at these positions precedes.
+    void ensure_coefficients() {
+        if (coef_ok || !n) return;
+        launch_density_alpha<Real>(ds, n, false, false, stream, true);
+        launches += 1;
+        coef_ok = true;
+    }
+
     // cuda_divergenceSolve (DFSPH_core_cuda.cu:785-861). lp: learned warm start (dfsph_step only).
     int divergence_solve(int max_iter, double max_error, bool lp = false) {
         if (!n) return DFSPH_OK;
         const double eta = max_error * 0.01 * sc.density0;  // divided by the device's h in the init pass
         if (!lp) {
-            launch_density_alpha<Real>(ds, n, true, false, stream);
+            density_pass(true, false);
             launch_divergence_warm_jacobi<Real>(ds, n, nullptr, nullptr, stream, boundary_forces);
             launch_divergence_residual<Real>(ds, n, true, eta, kMinItersV, max_iter, 0, false, stream);
             launches += 3;
         } else {
             const bool infer = mlp_ready && !base_only && net_useful, use = mlp_ready || base_only;
-            launch_density_alpha<Real>(ds, n, false, true, stream);
+            density_pass(false, true);
             if (infer) launch_mlp_forward(mlp, features, n, pred, status, stream);
             launch_warm_values<Real>(ds, n, 0, use, infer, damping, stream);
             launches += infer ? 3 : 2;
@@ -1700,6 +1730,7 @@ public:
     // cuda_update_vel is applied inside the warm-start pass.
     int pressure_solve(int max_iter, double max_error, bool fused_vel, bool lp = false) {
         if (!n) return DFSPH_OK;
+        ensure_coefficients();
         const double eta = max_error * 0.01 * sc.density0;
         if (!lp) {
             launch_pressure_warm_jacobi<Real>(ds, n, fused_vel, nullptr, nullptr, stream, boundary_forces);
@@ -1729,6 +1760,7 @@ public:
 
     int external_forces(bool cfl) {
         if (!n) return DFSPH_OK;
+        ensure_coefficients();
         launch_viscosity<Real>(ds, n, cfl, stream);
         launches += 1;
         vel_updated = false;
@@ -1777,6 +1809,7 @@ public:
     int update_pos() {
         if (!n) return DFSPH_OK;
         launch_update_pos<Real>(ds, n, stream);
+        coef_ok = false;
         launches += 1;
         DF_CUDA(cudaGetLastError());
         return DFSPH_OK;
@@ -1875,7 +1908,7 @@ public:
         if (div) {
             DF_TRY(divergence_solve(sc.max_iterations_v, sc.max_error_v, lp));
         } else if (n) {
-            launch_density_alpha<Real>(ds, n, false, lp, stream);
+            density_pass(false, lp);
             launches += 1;
             if (lp) {  // no divergence solve: its warm-start arrays stay zero
                 DF_CUDA(cudaMemsetAsync(kappaVW, 0, (size_t)n * sizeof(Real), stream));
@@ -2696,7 +2729,7 @@ public:
         DF_CHECK(cnt_out && lists_out, DFSPH_E_INVALID, "null output");
         DF_CHECK(row >= cap, DFSPH_E_INVALID, "row length smaller than neighbor_capacity");
         if (!n) return DFSPH_OK;
-        std::vector<uint32_t> c(n), t((size_t)cap * stride), ids(n), bids(std::max<uint32_t>(nb, 1));
+        std::vector<uint32_t> c(n), t(4 * (size_t)group_capacity(cap) * stride), ids(n), bids(std::max<uint32_t>(nb, 1));
         DF_CUDA(cudaMemcpyAsync(c.data(), counts, n * sizeof(uint32_t), cudaMemcpyDeviceToHost, stream));
         DF_CUDA(cudaMemcpyAsync(t.data(), nbr, t.size() * sizeof(uint32_t), cudaMemcpyDeviceToHost, stream));
         DF_CUDA(cudaMemcpyAsync(ids.data(), id[cur], n * sizeof(uint32_t), cudaMemcpyDeviceToHost, stream));
@@ -2708,7 +2741,7 @@ public:
             cnt_out[2 * (size_t)me] = nf;
             cnt_out[2 * (size_t)me + 1] = nbc;
             for (uint32_t k = 0; k < nf + nbc && k < cap; ++k) {
-                const uint32_t j = t[(size_t)k * stride + i];
+                const uint32_t j = t[slot_word(k < nf ? k : 4u * slot_groups(nf) + (k - nf), stride, i)];
                 lists_out[(size_t)me * row + k] = (k < nf) ? ids[j] : bids[j];
             }
         }
@@ -2915,8 +2948,8 @@ public:
 
     void launch_kernel(int k) {
         switch (k) {
-            case DFSPH_K_NEIGHBOR_BUILD: launch_build_neighbors<Real>(ds, n, ftab, btab, stream, bshifted); break;
-            case DFSPH_K_DENSITY_ALPHA: launch_density_alpha<Real>(ds, n, false, false, stream); break;
+            case DFSPH_K_NEIGHBOR_BUILD: launch_build_neighbors<Real>(ds, n, ftab, btab, bnear, stream, bshifted); break;
+            case DFSPH_K_DENSITY_ALPHA: density_pass(false, false); break;
             case DFSPH_K_DIVERGENCE_JACOBI: launch_divergence_jacobi<Real>(ds, n, 0, false, stream); break;
             case DFSPH_K_DIVERGENCE_RESIDUAL:
                 launch_divergence_residual<Real>(ds, n, false, 0.0, 0, 0, 0, false, stream);
@@ -2929,7 +2962,10 @@ public:
                 launch_pressure_residual<Real>(ds, n, false, 0.0, 0, 0, 0, false, stream);
                 break;
             case DFSPH_K_PRESSURE_JACOBI: launch_pressure_jacobi<Real>(ds, n, 0, false, stream); break;
-            case DFSPH_K_UPDATE_POS: launch_update_pos<Real>(ds, n, stream); break;
+            case DFSPH_K_UPDATE_POS:
+                launch_update_pos<Real>(ds, n, stream);
+                coef_ok = false;
+                break;
             default: break;
         }
         launches += 1;
@@ -2940,6 +2976,7 @@ public:
         DF_CHECK(k >= 0 && k < DFSPH_K_COUNT && reps > 0, DFSPH_E_INVALID, "bad kernel id or reps");
         DF_CHECK(n > 0, DFSPH_E_STATE, "no fluid");
         double total = 0.0;
+        ensure_coefficients();
         for (int r = 0; r < reps; ++r) {
             DF_CUDA(cudaEventRecord(ev0, stream));
             if (k == DFSPH_K_SORT_REORDER) {

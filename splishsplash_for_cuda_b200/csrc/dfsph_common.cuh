@@ -86,6 +86,15 @@ template <class Real> using Vec4 = typename Vec4Traits<Real>::type;
 template <class Real> __device__ __forceinline__ Vec4<Real> ld4(const Vec4<Real>* p) { return *p; }
 template <> __device__ __forceinline__ float4 ld4<float>(const float4* p) { return __ldg(p); }
 
+// Products and dot products with fixed rounding: the compiler may contract a * b + c into an FMA or
+// not, depending on the code around it; passes that must agree bit for bit use these.
+__device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
+template <class Real>
+__device__ __forceinline__ Real dot3(Real ax, Real ay, Real az, Real bx, Real by, Real bz) {
+    return fma(az, bz, fma(ax, bx, mul_rn(ay, by)));
+}
+
 // ---------------------------------------------------------------------------------------------
 // Compensated (Kahan) accumulation of FP32 sums. For double the same code runs; the compensation
 // term is simply tiny.
@@ -93,6 +102,13 @@ template <class Real> struct KSum {
     Real s = Real(0), c = Real(0);
     __device__ __forceinline__ void add(Real v) {
         const Real y = v - c;
+        const Real t = s + y;
+        c = (t - s) - y;
+        s = t;
+    }
+    // Adds a * b; the product enters the compensated step unrounded (one FMA).
+    __device__ __forceinline__ void add_product(Real a, Real b) {
+        const Real y = fma(a, b, -c);
         const Real t = s + y;
         c = (t - s) - y;
         s = t;
@@ -114,6 +130,11 @@ template <class Real> struct NSum {
 template <class Real> struct KSum3 {
     KSum<Real> x, y, z;
     __device__ __forceinline__ void add(Real a, Real b, Real d) { x.add(a); y.add(b); z.add(d); }
+    __device__ __forceinline__ void add_product(Real f, Real a, Real b, Real d) {
+        x.add_product(f, a);
+        y.add_product(f, b);
+        z.add_product(f, d);
+    }
 };
 
 // ---------------------------------------------------------------------------------------------
@@ -210,147 +231,166 @@ template <class Real> struct Cubic {
         const Real q = r2 * rsqrt_(r2) * invH;
         return W_of_q(q);
     }
-    __device__ __forceinline__ void gradW(Real rx, Real ry, Real rz, Real& gx, Real& gy, Real& gz) const {
+    // f with grad W(r) = f r (0 for |r| <= 1e-6 and beyond the support).
+    __device__ __forceinline__ Real grad_factor(Real rx, Real ry, Real rz) const {
         const Real r2 = rx * rx + ry * ry + rz * rz;
-        gx = gy = gz = Real(0);
+        Real f = Real(0);
         if (r2 > Real(1e-12)) {
             const Real inv_rl = rsqrt_(r2);
             const Real q = r2 * inv_rl * invH;
             if (q <= Real(1)) {
                 const Real c = (q <= Real(0.5)) ? l * q * (Real(3) * q - Real(2)) : l * (-(Real(1) - q) * (Real(1) - q));
-                const Real f = c * inv_rl * invH;
-                gx = f * rx;
-                gy = f * ry;
-                gz = f * rz;
+                f = c * inv_rl * invH;
             }
         }
+        return f;
     }
-    __device__ __forceinline__ void W_gradW(Real rx, Real ry, Real rz, Real& w, Real& gx, Real& gy, Real& gz) const {
-        const Real r2 = rx * rx + ry * ry + rz * rz;
-        gx = gy = gz = Real(0);
-        w = W0;
-        if (r2 > Real(1e-12)) {
-            const Real inv_rl = rsqrt_(r2);
-            const Real q = r2 * inv_rl * invH;
-            w = W_of_q(q);
-            if (q <= Real(1)) {
-                const Real c = (q <= Real(0.5)) ? l * q * (Real(3) * q - Real(2)) : l * (-(Real(1) - q) * (Real(1) - q));
-                const Real f = c * inv_rl * invH;
-                gx = f * rx;
-                gy = f * ry;
-                gz = f * rz;
-            }
-        }
+    // The same with every rounding explicit: the compiler contracts grad_factor's multiplications and
+    // additions into FMAs differently from kernel to kernel. The solver passes use this one (as pair
+    // coefficients), whose bits are those the passes got when each evaluated the kernel itself; the
+    // density pass keeps grad_factor for its own sums for the same reason, because the sign of its
+    // divergence source switches the warm start of a particle on or off.
+    __device__ __forceinline__ Real pair_factor(Real rx, Real ry, Real rz) const {
+        const Real r2 = dot3(rx, ry, rz, rx, ry, rz);
+        const Real inv_rl = rsqrt_(r2);
+        const Real q = mul_rn(mul_rn(r2, inv_rl), invH);
+        const Real g = Real(1) - q;
+        const Real c = (q <= Real(0.5)) ? mul_rn(mul_rn(l, q), fma(Real(3), q, Real(-2))) : mul_rn(l, mul_rn(-g, g));
+        const Real f = mul_rn(mul_rn(c, inv_rl), invH);
+        return (r2 > Real(1e-12) && q <= Real(1)) ? f : Real(0);
     }
 };
 
 // ---------------------------------------------------------------------------------------------
-// Density terms m_j W_ij of the FP32 build in double-float arithmetic (unevaluated pairs of FP32
-// values, hi + lo, built from error-free transformations: Knuth's TwoSum, Dekker's Fast2Sum and
-// the FMA product error). Why: the density deviation rho - rho0 that drives the pressure solve is
-// ~1/40 of rho at the most compressed particles, and a plain FP32 term m_j W(q) carries ~5 ulp of
-// error (|r|^2 rounding, sqrt and the steep cubic amplify it), i.e. ~1e-4 kg/m^3 on rho and ~4e-6
-// relative on rho - rho0, kappa and the velocities it corrects. Forming |r|^2, q, W and m W as
-// pairs keeps each term within ~2^-40 of the exact value for the given FP32 coordinates; the sum
-// itself stays an FP32 compensated sum (hi parts in Neumaier's sum, lo parts in a plain FP32 sum).
-// Every operation is an explicit round-to-nearest intrinsic so nothing is contracted.
-// Density term m_j W(r_ij) of the FP32 build, evaluated in native FP64 from the FP32 distance
-// components (their squares are exact in FP64): the FP32 build sums rho - rho0 in FP64 from these
-// terms, so the density residual keeps the accuracy of the FP64 build where rho ~ rho0 cancels.
-// The self term (r = 0) is m k.
-// Every FP64 operation is rounded on its own (no contraction), in the order the oracle's FP32
-// instance evaluates it, so the two agree bit for bit on the same inputs.
+// Density term m_j W(r_ij) of the FP32 build, evaluated in FP64 from the FP32 distance components: the
+// density deviation rho - rho0 that drives the pressure solve is ~1/40 of rho at the most compressed
+// particles, and a plain FP32 term carries ~5 ulp of error (|r|^2 rounding, sqrt and the steep cubic
+// amplify it), i.e. ~4e-6 relative on rho - rho0, kappa and the velocities it corrects. The FP32 build
+// sums rho - rho0 in FP64 from these terms.
+// q = sqrt(q2) comes from the FP32 reciprocal square root and two Newton steps (Heron's method in its
+// division-free form, relative error 2^-22 -> 2^-44 -> rounding) instead of the correctly rounded FP64
+// square root: density pass 240 -> 205 us at 1 M particles, the stored densities of 27 k to 150 k
+// particles bit for bit the same. The self term (r = 0) is m k.
 __device__ __forceinline__ double density_term(const Cubic<float>& K, float rx, float ry, float rz, float m) {
     const double dx = rx, dy = ry, dz = rz;
-    const double r2 = __dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz));
-    const double q2 = __dmul_rn(r2, K.ih2_d);
+    const double q2 = fma(dz, dz, fma(dy, dy, dx * dx)) * K.ih2_d;
     if (q2 > 1.0) return 0.0;
-    double w = K.k_d;
-    if (q2 > 0.0) {
-        const double q = __dsqrt_rn(q2);
-        if (q <= 0.5) {
-            w = __dmul_rn(K.k_d, __dadd_rn(1.0, __dmul_rn(__dmul_rn(6.0, q2), __dadd_rn(q, -1.0))));
-        } else {
-            const double f = __dadd_rn(1.0, -q);
-            w = __dmul_rn(__dmul_rn(2.0, K.k_d), __dmul_rn(__dmul_rn(f, f), f));
-        }
+    double w = 1.0;        // W / k; 1 to the last bit below q2 = 1e-20
+    if (q2 > 1e-20) {
+        const double y = (double)rsqrtf((float)q2), hy = 0.5 * y;
+        double q = q2 * y;
+        q = fma(hy, fma(-q, q, q2), q);
+        q = fma(hy, fma(-q, q, q2), q);
+        const double f = 1.0 - q;
+        w = q <= 0.5 ? fma(-6.0 * q2, f, 1.0) : 2.0 * f * (f * f);
     }
-    return __dmul_rn(w, (double)m);
+    return w * (K.k_d * (double)m);
 }
 
 // ---------------------------------------------------------------------------------------------
-// Batched neighbour visit. The neighbours [k0, k1) of particle i are taken kGatherBatch at a time:
-// first the batch's indices are loaded (coalesced rows of the interleaved table), then load(u, j)
-// issues every gather of the batch, then use(u) consumes them in list order. Keeping a batch of
-// independent gathers in flight per thread hides the latency that a one-at-a-time loop exposes,
-// while the summation order (and so every result bit) stays that of the plain loop. Slots past the
-// end of the list load `fallback` (an in-range index) and are not used.
-#ifndef DFSPH_GATHER_BATCH
-#define DFSPH_GATHER_BATCH 4
-#endif
-constexpr int kGatherBatch = DFSPH_GATHER_BATCH;
-#ifndef DFSPH_PREFETCH_IDX
-#define DFSPH_PREFETCH_IDX 1
-#endif
-constexpr uint32_t kNoNeighbor = 0xFFFFFFFFu;
-// The neighbour-index stream (read once per pass, coalesced: 128 B per warp and list slot, no reuse)
-// is read through the read-only path without allocating in L1 (L1::no_allocate), so that the lines it
-// would take stay with the neighbours' positions and velocities, which the passes re-read from L1.
-// Measured per step: 2.9 % faster at 1 M particles (passes larger than L2), 2.2 % slower at 250 k
-// (L2-resident passes); a runtime choice by size cost more in registers than it saved. The asm is
-// volatile: a load hoisted out of its condition would read past the list.
-#ifndef DFSPH_IDX_NO_ALLOCATE
-#define DFSPH_IDX_NO_ALLOCATE 1
-#endif
-__device__ __forceinline__ uint32_t ld_idx(const uint32_t* p) {
-#if DFSPH_IDX_NO_ALLOCATE
-    uint32_t v;
-    asm volatile("ld.global.nc.L1::no_allocate.u32 %0, [%1];" : "=r"(v) : "l"(p));
-    return v;
-#else
-    return __ldg(p);
-#endif
+// Neighbour lists. A particle's list is a sequence of slots, the fluid neighbours first, then the
+// boundary neighbours from the next multiple of four on; four consecutive slots of a particle form a
+// group, and the groups of all particles are interleaved: group g of particle i is the uint4
+// nbr[g * stride + i], so a warp reads a group with one coalesced 512-byte load. The fluid part is
+// filled up to a multiple of four with the particle's own index, the boundary part with its last
+// entry, so that the passes have no remainder loop.
+//
+// Pair coefficients. The positions do not change between a neighbour search and the position update,
+// so the pass that follows the search (density_alpha_kernel) stores f(r_ij) for every slot, where
+// grad W_ij = f r_ij (0 for a fill-up slot); the ~13 passes of the two solvers form grad W_ij =
+// f (x_i - x_j) without evaluating the kernel again. The
+// passes were bound by instruction issue and the L1 pipe, not by DRAM, so the 4 bytes per slot they
+// read more cost less than the ~40 instructions they save. Measured at 1 M particles, 31 neighbours:
+// residual pass 138 -> 128 us, Jacobi pass 115 -> 85 us, step 2.59 -> 2.24 ms with the neighbour
+// build's and the viscosity pass's share; at 250 k 0.797 -> 0.715 ms, at 27 k 0.348 -> 0.271 ms.
+__host__ __device__ inline uint32_t slot_groups(uint32_t entries) { return (entries + 3u) >> 2; }
+// Elements that the arrays of fluid and boundary positions have to spare after their capacity, so that
+// the neighbour build's batched loads may run past the last run.
+constexpr uint32_t kScanPad = 3;
+// Groups that a list of at most `cap` entries can need.
+__host__ __device__ inline uint32_t group_capacity(uint32_t cap) { return (cap + 6u) / 4u; }
+// Element of slot k of particle i in the interleaved table (as 4-byte words).
+__host__ __device__ inline size_t slot_word(uint32_t k, uint32_t stride, uint32_t i) {
+    return 4u * ((size_t)(k >> 2) * stride + i) + (k & 3u);
 }
 
-template <int B, class Load, class Use>
-__device__ __forceinline__ void visit_neighbors(const uint32_t* __restrict__ nbr, uint32_t stride, uint32_t i,
-                                                uint32_t k0, uint32_t k1, uint32_t fallback, Load&& load, Use&& use) {
-#if DFSPH_PREFETCH_IDX
-    // The index loads of the next batch are issued before the gathers of this one, so that their
-    // latency (a coalesced stream, usually from DRAM) overlaps the dependent gathers.
-    uint32_t jj[B];
-#pragma unroll
-    for (int u = 0; u < B; ++u) jj[u] = (k0 + u) < k1 ? ld_idx(nbr + (size_t)(k0 + u) * stride + i) : kNoNeighbor;
-    for (uint32_t kb = k0; kb < k1; kb += B) {
-        uint32_t jn[B];
-#pragma unroll
-        for (int u = 0; u < B; ++u) {
-            const uint32_t k = kb + B + u;
-            jn[u] = k < k1 ? ld_idx(nbr + (size_t)k * stride + i) : kNoNeighbor;
+// Index and coefficient groups are read once per pass, coalesced: they go through the read-only path
+// without allocating in L1 (L1::no_allocate), so that the lines they would take stay with the
+// neighbours' positions and velocities, which the passes re-read from L1. The asm is volatile: a load
+// hoisted out of its condition would read past the list.
+__device__ __forceinline__ uint4 ld_group(const uint4* p) {
+    uint4 v;
+    asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+                 : "l"(p));
+    return v;
+}
+__device__ __forceinline__ float4 ld_group(const float4* p) {
+    float4 v;
+    asm volatile("ld.global.nc.L1::no_allocate.v4.f32 {%0, %1, %2, %3}, [%4];"
+                 : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+                 : "l"(p));
+    return v;
+}
+__device__ __forceinline__ double4a ld_group(const double4a* p) { return *p; }
+
+template <class T> __device__ __forceinline__ auto component(const T& v, int u) {
+    return u == 0 ? v.x : u == 1 ? v.y : u == 2 ? v.z : v.w;
+}
+
+// Visits the slots of `groups` groups from idx / coef on, B (2 or 4) at a time: load(u, j) issues the
+// gathers of a batch, use(u, f) consumes them in slot order. Keeping a batch of independent gathers
+// in flight per thread hides the latency that a one-at-a-time loop exposes; the next group's index
+// and coefficients are loaded before this group's gathers.
+template <int B, class Real, class Load, class Use>
+__device__ __forceinline__ void visit_pairs(const uint4* __restrict__ idx, const Vec4<Real>* __restrict__ coef,
+                                            uint32_t stride, uint32_t groups, Load&& load, Use&& use) {
+    if (!groups) return;
+    uint4 j = ld_group(idx);
+    Vec4<Real> f = ld_group(coef);
+    while (true) {
+        idx += stride;
+        coef += stride;
+        const bool more = --groups != 0;
+        uint4 jn;
+        Vec4<Real> fn;
+        if (more) {
+            jn = ld_group(idx);
+            fn = ld_group(coef);
         }
 #pragma unroll
-        for (int u = 0; u < B; ++u) load(u, jj[u] == kNoNeighbor ? fallback : jj[u]);
+        for (int b = 0; b < 4; b += B) {
 #pragma unroll
-        for (int u = 0; u < B; ++u)
-            if (kb + u < k1) use(u);
+            for (int u = 0; u < B; ++u) load(u, component(j, b + u));
 #pragma unroll
-        for (int u = 0; u < B; ++u) jj[u] = jn[u];
-    }
-#else
-    for (uint32_t kb = k0; kb < k1; kb += B) {
-        uint32_t jj[B];
-#pragma unroll
-        for (int u = 0; u < B; ++u) {
-            const uint32_t k = kb + u;
-            jj[u] = k < k1 ? ld_idx(nbr + (size_t)k * stride + i) : kNoNeighbor;
+            for (int u = 0; u < B; ++u) use(u, component(f, b + u));
         }
-#pragma unroll
-        for (int u = 0; u < B; ++u) load(u, jj[u] == kNoNeighbor ? fallback : jj[u]);
-#pragma unroll
-        for (int u = 0; u < B; ++u)
-            if (kb + u < k1) use(u);
+        if (!more) break;
+        j = jn;
+        f = fn;
     }
-#endif
+}
+
+// Visits the `entries` slots of the groups from idx on, two at a time: load(u, j), then use(u) for the
+// slots that are entries (k < entries).
+template <class Load, class Use>
+__device__ __forceinline__ void visit_neighbors(const uint4* __restrict__ idx, uint32_t stride, uint32_t entries,
+                                                Load&& load, Use&& use) {
+    if (!entries) return;
+    uint4 j = ld_group(idx);
+    for (uint32_t k = 0; k < entries; k += 4) {
+        idx += stride;
+        uint4 jn;
+        if (k + 4 < entries) jn = ld_group(idx);
+#pragma unroll
+        for (int b = 0; b < 4; b += 2) {
+            load(0, component(j, b));
+            load(1, component(j, b + 1));
+            if (k + b < entries) use(0);
+            if (k + b + 1 < entries) use(1);
+        }
+        j = jn;
+    }
 }
 
 // ---------------------------------------------------------------------------------------------

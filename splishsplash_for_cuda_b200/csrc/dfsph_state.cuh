@@ -26,7 +26,9 @@ template <class Real> struct DevState {
     Real* kcoef;           // densityAdv * factor, the Jacobi coefficient read by neighbours
     Vec4<Real>* acc;       // non-pressure acceleration
     uint32_t* counts;      // fluid count | boundary count << 16
-    uint32_t* nbr;         // interleaved neighbour table nbr[k * nbr_stride + i]
+    uint4* nbr;            // interleaved neighbour lists, nbr[g * nbr_stride + i] (dfsph_common.cuh)
+    Vec4<Real>* coef;      // pair coefficients f of the lists at the current positions, same layout
+    Real* vol;             // m / rho, for the viscosity pass
     // boundary, cell-sorted order
     const Vec4<Real>* bpos;  // x, y, z, psi
     const Vec4<Real>* bvel;  // vx, vy, vz, (unused)
@@ -36,7 +38,7 @@ template <class Real> struct DevState {
     unsigned long long* bforce;
     // reductions and control
     double* partials;      // one FP64 partial per block
-    LoopCtl* ctl;          // [0] divergence loop, [1] pressure loop, [2] CFL / misc, [3] candidate probe
+    LoopCtl* ctl;          // [0] divergence loop, [1] pressure loop, [2] CFL / misc, [3] plain warm-start candidate
     double* dtd;           // dt history in FP64 (see DtSlot); the kernels read their Real copies in p
     uint32_t* status;      // [0] DFSPH_ST_* bits, [1] scratch, [2] learned warm start kept (bit 0 div, 1 pressure)
     float* cfl_partials;   // per-block max |v + a h|^2
@@ -49,7 +51,7 @@ template <class Real> struct DevState {
     Real* kappaVW;         // warm-start value used by this step's divergence solve
     Real* kappaP;          // plain (reference) pressure warm-start candidate
     Real* kappaVP;         // plain (reference) divergence warm-start candidate
-    Vec4<Real>* velP;      // velocities after the plain candidate's warm-start pass (probe)
+    Vec4<Real>* velP;      // velocities after the plain candidate's warm-start pass
     Real* resid;           // unclamped density residual of the last pressure pass (null: not kept)
     Real* residV;          // unclamped divergence residual of the last divergence pass (null: not kept)
     Real* dadvP;           // plain candidate's clamped init residual (both candidates in one pass)
@@ -75,13 +77,16 @@ void launch_reorder_pair(const uint32_t* perm, uint32_t n, const Real* a_in, con
                          Real* b_out, cudaStream_t s);
 void launch_cell_bounds(const uint32_t* sorted_keys, uint32_t n, int dim_x, int dim_y, int dim_z, uint2* table,
                         cudaStream_t s);
+// near_boundary[cell] = 1 for the cells within two cells of a boundary particle's (cleared by the caller).
+void launch_mark_near_boundary(const uint32_t* sorted_keys, uint32_t nb, int dim_x, int dim_y, int dim_z,
+                               uint8_t* near_boundary, cudaStream_t s);
 template <class Real>
 void launch_build_neighbors(const DevState<Real>* d, uint32_t n, const uint2* fluid_table, const uint2* boundary_table,
-                            cudaStream_t s, bool boundary_shifted = false);
+                            const uint8_t* near_boundary, cudaStream_t s, bool boundary_shifted = false);
 // Checked builds only (no-ops otherwise): particle 0's first list entry := value; the range check of
 // every list entry and count (DFSPH_ST_INDEX, the offending particle's list emptied).
-void launch_corrupt_first_neighbor(uint32_t* nbr, const uint32_t* counts, uint32_t value, cudaStream_t s);
-void launch_validate_neighbors(uint32_t* counts, const uint32_t* nbr, uint32_t n, uint32_t n_boundary, uint32_t stride,
+void launch_corrupt_first_neighbor(uint4* nbr, const uint32_t* counts, uint32_t value, cudaStream_t s);
+void launch_validate_neighbors(uint32_t* counts, const uint4* nbr, uint32_t n, uint32_t n_boundary, uint32_t stride,
                                uint32_t cap, uint32_t* status, cudaStream_t s);
 constexpr bool kCheckedBuild =
 #ifdef DFSPH_CHECKED
@@ -97,17 +102,16 @@ void launch_scatter_by_id(const uint32_t* id, uint32_t n, const Real* src, int c
                           cudaStream_t s);
 
 // ---- launch wrappers (solver.cu) ------------------------------------------------------------------
-// warm_v: scale kappa_v into the reference warm start; features: write the MLP inputs instead.
+// warm_v: scale kappa_v into the reference warm start; features: write the MLP inputs instead;
+// rows_only: write the pair coefficients and m / rho alone (for a pass that no density pass at these
+// positions precedes).
 template <class Real>
-void launch_density_alpha(const DevState<Real>* d, uint32_t n, bool warm_v, bool features, cudaStream_t s);
+void launch_density_alpha(const DevState<Real>* d, uint32_t n, bool warm_v, bool features, cudaStream_t s,
+                          bool rows_only = false);
 // kw: warm-start coefficients (null = kappa_v); vout: output velocities (null = in place).
 template <class Real>
 void launch_divergence_warm_jacobi(const DevState<Real>* d, uint32_t n, const Real* kw, Vec4<Real>* vout,
                                    cudaStream_t s, bool forces = false);
-// Sum of the divergence (which = 0) or density (which = 1) residual of velocities `vel`, into ctl[3]
-// (no other write): the initial residual of a warm-start candidate.
-template <class Real>
-void launch_probe_residual(const DevState<Real>* d, uint32_t n, int which, const Vec4<Real>* vel, cudaStream_t s);
 // Warm-start candidates: which = 0 divergence (kappa_v), 1 pressure (kappa). Writes the plain
 // (reference) candidate to kappaVP / kappaP and, when learned, the learned one to kappa_v + kappaVW /
 // kappaW (otherwise the plain one there too).
@@ -152,12 +156,6 @@ template <class Real>
 void launch_residual_dual(const DevState<Real>* d, uint32_t n, int which, double eta, int min_it, int max_it,
                           cudaStream_t s);
 template <class Real> void launch_select_candidate(const DevState<Real>* d, uint32_t n, int which, cudaStream_t s);
-// Fallback init pass of the learned warm start (which = 0 divergence, 1 pressure): if the plain
-// candidate's probed residual (ctl[3]) is below the learned candidate's init residual, installs the
-// plain candidate and redoes the init pass; otherwise records the learned one as kept (status[2]).
-template <class Real>
-void launch_fallback_residual(const DevState<Real>* d, uint32_t n, int which, double eta, int min_it, int max_it,
-                              cudaStream_t s);
 template <class Real>
 void launch_pressure_jacobi(const DevState<Real>* d, uint32_t n, cudaGraphConditionalHandle h, bool use_handle,
                             cudaStream_t s, bool forces = false);

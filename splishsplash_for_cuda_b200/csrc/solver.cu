@@ -22,12 +22,6 @@ namespace dfsph {
 
 namespace {
 
-// Neighbours per batch in the passes that carry both warm-start candidates.
-#ifndef DFSPH_DUAL_BATCH
-#define DFSPH_DUAL_BATCH 2
-#endif
-constexpr int kDualBatch = DFSPH_DUAL_BATCH;
-
 template <class Real> __device__ __forceinline__ Real rmax(Real a, Real b);
 template <> __device__ __forceinline__ float rmax<float>(float a, float b) { return fmaxf(a, b); }
 template <> __device__ __forceinline__ double rmax<double>(double a, double b) { return fmax(a, b); }
@@ -157,17 +151,19 @@ __device__ __forceinline__ void load_bnbr(BNbr<Real>& b, const Vec4<Real>* __res
     }
 }
 
-// Neighbours per gather batch of the residual passes (3) and the density pass (2): at four the
-// residual passes spill 16-24 B and the density pass (FP64 density terms) 276 B at the 64-register
-// cap. Measured per step against four: -0.3 % / -0.8 % at 1 M particles, -1.2 % each at 250 k.
-#ifndef DFSPH_RESID_BATCH
-#define DFSPH_RESID_BATCH 3
+// Slots whose gathers are in flight at a time in the single-candidate solver loops (two in the others,
+// which carry more state per thread).
+#ifndef DFSPH_PAIR_BATCH
+#define DFSPH_PAIR_BATCH 4
 #endif
-constexpr int kResidBatch = DFSPH_RESID_BATCH;
-#ifndef DFSPH_DENSITY_BATCH
-#define DFSPH_DENSITY_BATCH 2
-#endif
-constexpr int kDensityBatch = DFSPH_DENSITY_BATCH;
+constexpr int kPairBatch = DFSPH_PAIR_BATCH;
+
+// One term m_j (v_i - v_j).grad W_ij of a divergence, grad W_ij = f (x_i - x_j).
+template <class Real>
+__device__ __forceinline__ void add_divergence(KSum<Real>& s, Real m, Real f, Real rx, Real ry, Real rz, Real dvx, Real dvy,
+                                               Real dvz) {
+    s.add_product(m, dot3(dvx, dvy, dvz, mul_rn(f, rx), mul_rn(f, ry), mul_rn(f, rz)));
+}
 
 // Sum over fluid then boundary neighbours of m_j (v_i - v_j).grad W_ij, in list order.
 template <class Real>
@@ -175,38 +171,40 @@ __device__ __forceinline__ Real velocity_divergence(const DevState<Real>* __rest
                                                     uint32_t i, const Vec4<Real>& xi, const Vec4<Real>& vi,
                                                     uint32_t nf, uint32_t nb, const Vec4<Real>* __restrict__ vel) {
     const Vec4<Real>* __restrict__ pos = ds->pos;
-    const uint32_t* __restrict__ nbr = ds->nbr;
     const uint32_t stride = p.nbr_stride;
-    const Cubic<Real> K = p.kern;
+    const uint4* __restrict__ idx = ds->nbr + i;
+    const Vec4<Real>* __restrict__ coef = ds->coef + i;
     KSum<Real> s;
-    Vec4<Real> xj[kResidBatch], vj[kResidBatch];
-    visit_neighbors<kResidBatch>(
-        nbr, stride, i, 0, nf, i,
-        [&](int u, uint32_t j) {
-            xj[u] = ld4<Real>(pos + j);
-            vj[u] = ld4<Real>(vel + j);
-        },
-        [&](int u) {
-            Real gx, gy, gz;
-            K.gradW(xi.x - xj[u].x, xi.y - xj[u].y, xi.z - xj[u].z, gx, gy, gz);
-            s.add(xj[u].w * ((vi.x - vj[u].x) * gx + (vi.y - vj[u].y) * gy + (vi.z - vj[u].z) * gz));
-        });
+    {
+        Vec4<Real> xj[kPairBatch], vj[kPairBatch];
+        visit_pairs<kPairBatch, Real>(
+            idx, coef, stride, slot_groups(nf),
+            [&](int u, uint32_t j) {
+                xj[u] = ld4<Real>(pos + j);
+                vj[u] = ld4<Real>(vel + j);
+            },
+            [&](int u, Real f) {
+                add_divergence(s, xj[u].w, f, xi.x - xj[u].x, xi.y - xj[u].y, xi.z - xj[u].z, vi.x - vj[u].x,
+                               vi.y - vj[u].y, vi.z - vj[u].z);
+            });
+    }
     if (nb) {
         const bool moving = p.boundary_moving != 0;
-        BNbr<Real> b[kResidBatch];
-        visit_neighbors<kResidBatch>(
-            nbr, stride, i, nf, nf + nb, 0u, [&](int u, uint32_t j) { load_bnbr(b[u], ds->bpos, ds->bvel, j, moving); },
-            [&](int u) {
-                Real gx, gy, gz;
-                K.gradW(xi.x - b[u].x.x, xi.y - b[u].x.y, xi.z - b[u].x.z, gx, gy, gz);
-                s.add(b[u].x.w * ((vi.x - b[u].vx) * gx + (vi.y - b[u].vy) * gy + (vi.z - b[u].vz) * gz));
+        const size_t at = (size_t)slot_groups(nf) * stride;
+        BNbr<Real> b[2];
+        visit_pairs<2, Real>(
+            idx + at, coef + at, stride, slot_groups(nb),
+            [&](int u, uint32_t j) { load_bnbr(b[u], ds->bpos, ds->bvel, j, moving); },
+            [&](int u, Real f) {
+                add_divergence(s, b[u].x.w, f, xi.x - b[u].x.x, xi.y - b[u].x.y, xi.z - b[u].x.z, vi.x - b[u].vx,
+                               vi.y - b[u].vy, vi.z - b[u].vz);
             });
     }
     return s.value();
 }
 
-// velocity_divergence for two velocity fields in one pass over the neighbours (positions and
-// indices loaded once); each sum is accumulated exactly as velocity_divergence would.
+// velocity_divergence for two velocity fields in one pass over the neighbours (positions, indices and
+// coefficients loaded once); each sum is accumulated exactly as velocity_divergence would.
 template <class Real>
 __device__ __forceinline__ void velocity_divergence2(const DevState<Real>* __restrict__ ds, const StepParams<Real>& p,
                                                      uint32_t i, const Vec4<Real>& xi, const Vec4<Real>& via,
@@ -214,94 +212,104 @@ __device__ __forceinline__ void velocity_divergence2(const DevState<Real>* __res
                                                      const Vec4<Real>* __restrict__ vela,
                                                      const Vec4<Real>* __restrict__ velb, Real& outa, Real& outb) {
     const Vec4<Real>* __restrict__ pos = ds->pos;
-    const uint32_t* __restrict__ nbr = ds->nbr;
     const uint32_t stride = p.nbr_stride;
-    const Cubic<Real> K = p.kern;
+    const uint4* __restrict__ idx = ds->nbr + i;
+    const Vec4<Real>* __restrict__ coef = ds->coef + i;
     KSum<Real> sa, sb;
-    Vec4<Real> xj[kDualBatch], va[kDualBatch], vb[kDualBatch];
-    visit_neighbors<kDualBatch>(
-        nbr, stride, i, 0, nf, i,
-        [&](int u, uint32_t j) {
-            xj[u] = ld4<Real>(pos + j);
-            va[u] = ld4<Real>(vela + j);
-            vb[u] = ld4<Real>(velb + j);
-        },
-        [&](int u) {
-            Real gx, gy, gz;
-            K.gradW(xi.x - xj[u].x, xi.y - xj[u].y, xi.z - xj[u].z, gx, gy, gz);
-            sa.add(xj[u].w * ((via.x - va[u].x) * gx + (via.y - va[u].y) * gy + (via.z - va[u].z) * gz));
-            sb.add(xj[u].w * ((vib.x - vb[u].x) * gx + (vib.y - vb[u].y) * gy + (vib.z - vb[u].z) * gz));
-        });
+    {
+        Vec4<Real> xj[2], va[2], vb[2];
+        visit_pairs<2, Real>(
+            idx, coef, stride, slot_groups(nf),
+            [&](int u, uint32_t j) {
+                xj[u] = ld4<Real>(pos + j);
+                va[u] = ld4<Real>(vela + j);
+                vb[u] = ld4<Real>(velb + j);
+            },
+            [&](int u, Real f) {
+                const Real rx = xi.x - xj[u].x, ry = xi.y - xj[u].y, rz = xi.z - xj[u].z;
+                add_divergence(sa, xj[u].w, f, rx, ry, rz, via.x - va[u].x, via.y - va[u].y, via.z - va[u].z);
+                add_divergence(sb, xj[u].w, f, rx, ry, rz, vib.x - vb[u].x, vib.y - vb[u].y, vib.z - vb[u].z);
+            });
+    }
     if (nb) {
         const bool moving = p.boundary_moving != 0;
-        BNbr<Real> b[kDualBatch];
-        visit_neighbors<kDualBatch>(
-            nbr, stride, i, nf, nf + nb, 0u, [&](int u, uint32_t j) { load_bnbr(b[u], ds->bpos, ds->bvel, j, moving); },
-            [&](int u) {
-                Real gx, gy, gz;
-                K.gradW(xi.x - b[u].x.x, xi.y - b[u].x.y, xi.z - b[u].x.z, gx, gy, gz);
-                sa.add(b[u].x.w * ((via.x - b[u].vx) * gx + (via.y - b[u].vy) * gy + (via.z - b[u].vz) * gz));
-                sb.add(b[u].x.w * ((vib.x - b[u].vx) * gx + (vib.y - b[u].vy) * gy + (vib.z - b[u].vz) * gz));
+        const size_t at = (size_t)slot_groups(nf) * stride;
+        BNbr<Real> b[2];
+        visit_pairs<2, Real>(
+            idx + at, coef + at, stride, slot_groups(nb),
+            [&](int u, uint32_t j) { load_bnbr(b[u], ds->bpos, ds->bvel, j, moving); },
+            [&](int u, Real f) {
+                const Real rx = xi.x - b[u].x.x, ry = xi.y - b[u].x.y, rz = xi.z - b[u].x.z;
+                add_divergence(sa, b[u].x.w, f, rx, ry, rz, via.x - b[u].vx, via.y - b[u].vy, via.z - b[u].vz);
+                add_divergence(sb, b[u].x.w, f, rx, ry, rz, vib.x - b[u].vx, vib.y - b[u].vy, vib.z - b[u].vz);
             });
     }
     outa = sa.value();
     outb = sb.value();
 }
 
+// Boundary part of a Jacobi sum: use(j, psi_b, grad W_ib) for every boundary neighbour (b = j).
+template <class Real, class Use>
+__device__ __forceinline__ void visit_boundary(const DevState<Real>* __restrict__ ds, uint32_t stride, uint32_t i,
+                                               const Vec4<Real>& xi, uint32_t nf, uint32_t nb, Use&& use) {
+    const Vec4<Real>* __restrict__ bpos = ds->bpos;
+    Vec4<Real> xb[2];
+    uint32_t jb[2];
+    const size_t at = (size_t)slot_groups(nf) * stride + i;
+    visit_pairs<2, Real>(
+        ds->nbr + at, ds->coef + at, stride, slot_groups(nb),
+        [&](int u, uint32_t j) {
+            xb[u] = ld4<Real>(bpos + j);
+            jb[u] = j;
+        },
+        [&](int u, Real f) {
+            use(jb[u], xb[u].w, mul_rn(f, xi.x - xb[u].x), mul_rn(f, xi.y - xb[u].y), mul_rn(f, xi.z - xb[u].z));
+        });
+}
+// The reaction f grad W_ib on boundary particle j, as the reference adds it for dynamic bodies
+// (DFSPH_core_cuda.cu:467-477, :937-946).
+template <class Real>
+__device__ __forceinline__ void add_boundary_force(unsigned long long* bf, uint32_t j, Real f, Real gx, Real gy, Real gz) {
+    unsigned long long* fb = bf + 3 * (size_t)j;
+    add_force_fx(fb, (double)(f * gx));
+    add_force_fx(fb + 1, (double)(f * gy));
+    add_force_fx(fb + 2, (double)(f * gz));
+}
+
 // Jacobi velocity correction: sum over fluid neighbours of (k_i + k_j) m_j grad W_ij where
 // |k_i + k_j| > eps, plus (when |k_i| > eps) k_i sum over boundary neighbours of psi_b grad W_ib.
-// kof(j) returns k_j (a load, possibly transformed). With boundary forces on (kForces, and at run
-// time `forces`), each boundary term also adds -m_i k_i psi_b grad W_ib to the boundary particle's force,
-// as the reference does for dynamic bodies (DFSPH_core_cuda.cu:467-477, :937-946).
+// kof(j) returns k_j (a load, possibly transformed). With boundary forces on (kForces, and at run time
+// `forces`), each boundary term also adds -m_i k_i psi_b grad W_ib to the boundary particle's force.
+// A fill-up slot (f = 0) adds a zero and leaves the sum as it is.
 template <class Real, bool kForces = false, class KOf>
 __device__ __forceinline__ void jacobi_sum(const DevState<Real>* __restrict__ ds, const StepParams<Real>& p, uint32_t i,
                                            const Vec4<Real>& xi, Real ki, uint32_t nf, uint32_t nb, KOf&& kof,
                                            KSum3<Real>& acc, bool forces = true) {
     const Vec4<Real>* __restrict__ pos = ds->pos;
-    const uint32_t* __restrict__ nbr = ds->nbr;
     const uint32_t stride = p.nbr_stride;
-    const Cubic<Real> K = p.kern;
-    Vec4<Real> xj[kGatherBatch];
-    Real kj[kGatherBatch];
-    visit_neighbors<kGatherBatch>(
-        nbr, stride, i, 0, nf, i,
-        [&](int u, uint32_t j) {
-            xj[u] = ld4<Real>(pos + j);
-            kj[u] = kof(j);
-        },
-        [&](int u) {
-            const Real ks = ki + kj[u];
-            if (above_eps(ks)) {
-                Real gx, gy, gz;
-                K.gradW(xi.x - xj[u].x, xi.y - xj[u].y, xi.z - xj[u].z, gx, gy, gz);
-                const Real sc = ks * xj[u].w;
-                acc.add(sc * gx, sc * gy, sc * gz);
-            }
-        });
-    if (nb && above_eps(ki)) {
-        const Vec4<Real>* __restrict__ bpos = ds->bpos;
-        unsigned long long* __restrict__ bf = (kForces && forces) ? ds->bforce : nullptr;
-        Vec4<Real> xb[kGatherBatch];
-        uint32_t jb[kGatherBatch];
-        visit_neighbors<kGatherBatch>(
-            nbr, stride, i, nf, nf + nb, 0u,
+    {
+        Vec4<Real> xj[kPairBatch];
+        Real kj[kPairBatch];
+        visit_pairs<kPairBatch, Real>(
+            ds->nbr + i, ds->coef + i, stride, slot_groups(nf),
             [&](int u, uint32_t j) {
-                xb[u] = ld4<Real>(bpos + j);
-                jb[u] = j;
+                xj[u] = ld4<Real>(pos + j);
+                kj[u] = kof(j);
             },
-            [&](int u) {
-                Real gx, gy, gz;
-                K.gradW(xi.x - xb[u].x, xi.y - xb[u].y, xi.z - xb[u].z, gx, gy, gz);
-                const Real sc = ki * xb[u].w;
-                acc.add(sc * gx, sc * gy, sc * gz);
-                if (kForces && bf) {
-                    const Real f = -xi.w * sc;
-                    unsigned long long* fb = bf + 3 * (size_t)jb[u];
-                    add_force_fx(fb, (double)(f * gx));
-                    add_force_fx(fb + 1, (double)(f * gy));
-                    add_force_fx(fb + 2, (double)(f * gz));
-                }
+            [&](int u, Real f) {
+                const Real ks = ki + kj[u];
+                if (above_eps(ks))
+                    acc.add_product(mul_rn(ks, xj[u].w), mul_rn(f, xi.x - xj[u].x), mul_rn(f, xi.y - xj[u].y),
+                                    mul_rn(f, xi.z - xj[u].z));
             });
+    }
+    if (nb && above_eps(ki)) {
+        unsigned long long* __restrict__ bf = (kForces && forces) ? ds->bforce : nullptr;
+        visit_boundary<Real>(ds, stride, i, xi, nf, nb, [&](uint32_t j, Real psi, Real gx, Real gy, Real gz) {
+            const Real sc = mul_rn(ki, psi);
+            acc.add_product(sc, gx, gy, gz);
+            if (kForces && bf) add_boundary_force(bf, j, -xi.w * sc, gx, gy, gz);
+        });
     }
 }
 
@@ -315,83 +323,79 @@ __device__ __forceinline__ void jacobi_sum2(const DevState<Real>* __restrict__ d
                                             uint32_t nb, KOfA&& kofa, KOfB&& kofb, KSum3<Real>& acca,
                                             KSum3<Real>& accb) {
     const Vec4<Real>* __restrict__ pos = ds->pos;
-    const uint32_t* __restrict__ nbr = ds->nbr;
     const uint32_t stride = p.nbr_stride;
-    const Cubic<Real> K = p.kern;
-    Vec4<Real> xj[kDualBatch];
-    Real kja[kDualBatch], kjb[kDualBatch];
-    visit_neighbors<kDualBatch>(
-        nbr, stride, i, 0, nf, i,
-        [&](int u, uint32_t j) {
-            xj[u] = ld4<Real>(pos + j);
-            kja[u] = kofa(j);
-            kjb[u] = kofb(j);
-        },
-        [&](int u) {
-            const Real ksa = kia + kja[u], ksb = kib + kjb[u];
-            const bool ea = above_eps(ksa), eb = above_eps(ksb);
-            if (ea || eb) {
-                Real gx, gy, gz;
-                K.gradW(xi.x - xj[u].x, xi.y - xj[u].y, xi.z - xj[u].z, gx, gy, gz);
-                if (ea) {
-                    const Real sc = ksa * xj[u].w;
-                    acca.add(sc * gx, sc * gy, sc * gz);
-                }
-                if (eb) {
-                    const Real sc = ksb * xj[u].w;
-                    accb.add(sc * gx, sc * gy, sc * gz);
-                }
-            }
-        });
+    {
+        Vec4<Real> xj[2];
+        Real kja[2], kjb[2];
+        visit_pairs<2, Real>(
+            ds->nbr + i, ds->coef + i, stride, slot_groups(nf),
+            [&](int u, uint32_t j) {
+                xj[u] = ld4<Real>(pos + j);
+                kja[u] = kofa(j);
+                kjb[u] = kofb(j);
+            },
+            [&](int u, Real f) {
+                const Real ksa = kia + kja[u], ksb = kib + kjb[u];
+                const Real gx = mul_rn(f, xi.x - xj[u].x), gy = mul_rn(f, xi.y - xj[u].y), gz = mul_rn(f, xi.z - xj[u].z);
+                if (above_eps(ksa)) acca.add_product(mul_rn(ksa, xj[u].w), gx, gy, gz);
+                if (above_eps(ksb)) accb.add_product(mul_rn(ksb, xj[u].w), gx, gy, gz);
+            });
+    }
     const bool ba = above_eps(kia), bb = above_eps(kib);
     if (nb && (ba || bb)) {
-        const Vec4<Real>* __restrict__ bpos = ds->bpos;
         unsigned long long* __restrict__ bf = kForces ? ds->bforce : nullptr;
-        Vec4<Real> xb[kDualBatch];
-        uint32_t jb[kDualBatch];
-        visit_neighbors<kDualBatch>(
-            nbr, stride, i, nf, nf + nb, 0u,
-            [&](int u, uint32_t j) {
-                xb[u] = ld4<Real>(bpos + j);
-                jb[u] = j;
-            },
-            [&](int u) {
-                Real gx, gy, gz;
-                K.gradW(xi.x - xb[u].x, xi.y - xb[u].y, xi.z - xb[u].z, gx, gy, gz);
-                if (ba) {
-                    const Real sc = kia * xb[u].w;
-                    acca.add(sc * gx, sc * gy, sc * gz);
-                }
-                if (bb) {
-                    const Real sc = kib * xb[u].w;
-                    accb.add(sc * gx, sc * gy, sc * gz);
-                    if (kForces && bf) {
-                        const Real f = -xi.w * sc;
-                        unsigned long long* fb = bf + 3 * (size_t)jb[u];
-                        add_force_fx(fb, (double)(f * gx));
-                        add_force_fx(fb + 1, (double)(f * gy));
-                        add_force_fx(fb + 2, (double)(f * gz));
-                    }
-                }
-            });
+        visit_boundary<Real>(ds, stride, i, xi, nf, nb, [&](uint32_t j, Real psi, Real gx, Real gy, Real gz) {
+            if (ba) acca.add_product(mul_rn(kia, psi), gx, gy, gz);
+            if (bb) {
+                const Real sc = mul_rn(kib, psi);
+                accb.add_product(sc, gx, gy, gz);
+                if (kForces && bf) add_boundary_force(bf, j, -xi.w * sc, gx, gy, gz);
+            }
+        });
+    }
+}
+
+// Visits the `entries` slots of the groups from idx on two at a time (load(u, j), then f = use(u)) and
+// writes their pair coefficients, 0 for the fill-up slots.
+template <class Real, class Load, class Use>
+__device__ __forceinline__ void visit_coefficients(const uint4* __restrict__ idx, Vec4<Real>* __restrict__ coef,
+                                                   uint32_t stride, uint32_t entries, Load&& load, Use&& use) {
+    if (!entries) return;
+    uint4 j = ld_group(idx);
+    for (uint32_t k = 0; k < entries; k += 4) {
+        idx += stride;
+        uint4 jn;
+        if (k + 4 < entries) jn = ld_group(idx);
+        Vec4<Real> f;
+        f.x = f.y = f.z = f.w = Real(0);
+        load(0, j.x);
+        load(1, j.y);
+        f.x = use(0);
+        if (k + 1 < entries) f.y = use(1);
+        load(0, j.z);
+        load(1, j.w);
+        if (k + 2 < entries) f.z = use(0);
+        if (k + 3 < entries) f.w = use(1);
+        *coef = f;
+        coef += stride;
+        j = jn;
     }
 }
 
 // ---------------------------------------------------------------------------------------------
 // density + alpha + divergence source (+ kappa_v warm-start scaling), one pass over the neighbours.
-// warm_v and features are runtime flags so that every mode runs the same machine code for the
-// density and alpha arithmetic (the learned mode with a plain warm start reproduces the plain mode
-// bit for bit).
+// warm_v, features and rows_only are runtime flags so that every mode runs the same machine code for
+// the density, alpha and pair arithmetic (the learned mode with a plain warm start reproduces the plain
+// mode bit for bit, and rebuilt coefficients are those of the density pass).
 template <class Real>
 __global__ void __launch_bounds__(kBlock, kGatherMinBlocks) density_alpha_kernel(const DevState<Real>* __restrict__ ds, uint32_t n,
-                                                                               bool warm_v, bool features) {
+                                                                               bool warm_v, bool features, bool rows_only) {
     DFSPH_PDL_ENTER;
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const StepParams<Real>& p = ds->p;
     const Vec4<Real>* __restrict__ pos = ds->pos;
     const Vec4<Real>* __restrict__ vel = ds->vel;
-    const uint32_t* __restrict__ nbr = ds->nbr;
     const uint32_t stride = p.nbr_stride;
     const Cubic<Real> K = p.kern;
 
@@ -420,33 +424,45 @@ __global__ void __launch_bounds__(kBlock, kGatherMinBlocks) density_alpha_kernel
         }
     };
     add_term(Real(0), Real(0), Real(0), xi.w, K.W0);
-    auto accumulate = [&](const Vec4<Real>& xj, Real vx, Real vy, Real vz) {
-        Real w, gx, gy, gz;
-        const Real rx = xi.x - xj.x, ry = xi.y - xj.y, rz = xi.z - xj.z;
-        if constexpr (kF64Terms) K.gradW(rx, ry, rz, gx, gy, gz), w = Real(0);
-        else K.W_gradW(rx, ry, rz, w, gx, gy, gz);
-        add_term(rx, ry, rz, xj.w, w);
+    auto accumulate = [&](const Vec4<Real>& xj, Real vx, Real vy, Real vz, Real rx, Real ry, Real rz, Real f) {
+        add_term(rx, ry, rz, xj.w, kF64Terms ? Real(0) : K.W(rx, ry, rz));
+        const Real gx = f * rx, gy = f * ry, gz = f * rz;
         const Real px = xj.w * gx, py = xj.w * gy, pz = xj.w * gz;
         sgk.add(px * px + py * py + pz * pz);
         gpi.add(px, py, pz);
         drho.add((vi.x - vx) * px + (vi.y - vy) * py + (vi.z - vz) * pz);
     };
     {
-        Vec4<Real> xj[kDensityBatch], vj[kDensityBatch];
-        visit_neighbors<kDensityBatch>(
-            nbr, stride, i, 0, nf, i,
+        Vec4<Real> xj[2], vj[2];
+        visit_coefficients<Real>(
+            ds->nbr + i, ds->coef + i, stride, nf,
             [&](int u, uint32_t j) {
                 xj[u] = ld4<Real>(pos + j);
                 vj[u] = ld4<Real>(vel + j);
             },
-            [&](int u) { accumulate(xj[u], vj[u].x, vj[u].y, vj[u].z); });
+            [&](int u) {
+                const Real rx = xi.x - xj[u].x, ry = xi.y - xj[u].y, rz = xi.z - xj[u].z;
+                accumulate(xj[u], vj[u].x, vj[u].y, vj[u].z, rx, ry, rz, K.grad_factor(rx, ry, rz));
+                return K.pair_factor(rx, ry, rz);
+            });
     }
     if (nb) {
         const bool moving = p.boundary_moving != 0;
-        BNbr<Real> b[kDensityBatch];
-        visit_neighbors<kDensityBatch>(
-            nbr, stride, i, nf, nf + nb, 0u, [&](int u, uint32_t j) { load_bnbr(b[u], ds->bpos, ds->bvel, j, moving); },
-            [&](int u) { accumulate(b[u].x, b[u].vx, b[u].vy, b[u].vz); });
+        BNbr<Real> b[2];
+        const size_t at = (size_t)slot_groups(nf) * stride + i;
+        visit_coefficients<Real>(
+            ds->nbr + at, ds->coef + at, stride, nb,
+            [&](int u, uint32_t j) { load_bnbr(b[u], ds->bpos, ds->bvel, j, moving); },
+            [&](int u) {
+                const Real rx = xi.x - b[u].x.x, ry = xi.y - b[u].x.y, rz = xi.z - b[u].x.z;
+                const Real f = K.pair_factor(rx, ry, rz);
+                accumulate(b[u].x, b[u].vx, b[u].vy, b[u].vz, rx, ry, rz, f);
+                return f;
+            });
+    }
+    if (rows_only) {
+        ds->vol[i] = xi.w / (p.density0 + ds->density[i]);
+        return;
     }
     const Real gx = gpi.x.value(), gy = gpi.y.value(), gz = gpi.z.value();
     const Real sg = sgk.value() + (gx * gx + gy * gy + gz * gz);
@@ -454,6 +470,7 @@ __global__ void __launch_bounds__(kBlock, kGatherMinBlocks) density_alpha_kernel
     const Real density = kF64Terms ? (Real)rho64 : rho.value();
     ds->factor[i] = alpha;
     ds->density[i] = density;
+    ds->vol[i] = xi.w / (p.density0 + density);
     uint32_t num = nf;
     if (num < kMinNeighborsForDivergence) num += nb;
     const Real dadv = (num < kMinNeighborsForDivergence) ? Real(0) : rmax<Real>(drho.value(), Real(0));
@@ -494,22 +511,8 @@ __global__ void __launch_bounds__(kBlock, kGatherMinBlocks) divergence_warm_jaco
     (vout ? vout : ds->vel)[i] = v;
 }
 
-// Residual pass modes: a loop iteration, the init pass, and the fallback init pass of the learned
-// warm start (runs only if the plain candidate's probed residual, ctl[3], beat the learned
-// candidate's init residual; it then installs the plain candidate: velocities from velP, warm
-// coefficients from the plain array, and redoes the init on them).
-constexpr int kLoop = 0, kInitPass = 1, kFallback = 2;
-
-// True in every block of a fallback pass when the plain candidate is to replace the learned one:
-// when the learned candidate's sum |r| (its init pass, ctl[slot].aux) exceeds the plain one's
-// (probe, ctl[3].sum). Both sums are final before the launch; a NaN also falls back.
-template <class Real>
-__device__ __forceinline__ bool take_fallback(const DevState<Real>* __restrict__ ds, int slot, uint32_t bit) {
-    const double plain = ds->ctl[3].sum, learned = ds->ctl[slot].aux;
-    const bool fb = !(learned <= plain);
-    if (!fb && blockIdx.x == 0 && threadIdx.x == 0) atomicOr(ds->status + 2, bit);
-    return fb;
-}
+// Residual pass modes: a loop iteration and the init pass.
+constexpr int kLoop = 0, kInitPass = 1;
 
 // Divergence residual (computeDensityChange): rho_dot_i = max(sum m_j (v_i - v_j).grad W_ij +
 // sum psi_b (v_i - v_b).grad W_ib, 0), 0 with fewer than 20 neighbours. Also stores
@@ -524,17 +527,12 @@ __global__ void __launch_bounds__(kBlock, kGatherMinBlocks) divergence_residual_
     // The init passes receive the tolerance per unit of h (maxErrorV 0.01 rho0 / h): h is the
     // device's (the dt history lives on the device).
     if (kMode != kLoop) eta = eta / ds->dtd[kDtH];
-    if (kMode == kFallback && !take_fallback(ds, 0, 1u)) return;  // uniform over the grid
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    const Vec4<Real>* __restrict__ vel = kMode == kFallback ? ds->velP : ds->vel;
+    const Vec4<Real>* __restrict__ vel = ds->vel;
     double contrib = 0.0, aux = 0.0;
     if (i < n) {
         const StepParams<Real>& p = ds->p;
         if (kMode != kLoop) ds->kappaV[i] = Real(0);
-        if (kMode == kFallback) {
-            ds->vel[i] = vel[i];
-            ds->kappaVW[i] = ds->kappaVP[i];
-        }
         const uint32_t c = ds->counts[i];
         const uint32_t nf = fluid_count(c), nb = boundary_count(c);
         uint32_t num = nf;
@@ -589,10 +587,6 @@ __global__ void __launch_bounds__(kBlock, kGatherMinBlocks) divergence_jacobi_ke
 // neighbours. With kCfl the block maximum of |v + a h|^2 is stored for the CFL time step.
 // The viscosity pass gathers position, velocity and density: at four neighbours per batch it spills
 // at the 64-register cap; two per batch runs without spills, 14 % faster at 1 M particles.
-#ifndef DFSPH_VISC_BATCH
-#define DFSPH_VISC_BATCH 2
-#endif
-constexpr int kViscBatch = DFSPH_VISC_BATCH;
 template <class Real, bool kCfl>
 __global__ void __launch_bounds__(kBlock, kGatherMinBlocks) viscosity_kernel(const DevState<Real>* __restrict__ ds, uint32_t n) {
     DFSPH_PDL_ENTER;
@@ -602,25 +596,25 @@ __global__ void __launch_bounds__(kBlock, kGatherMinBlocks) viscosity_kernel(con
         const StepParams<Real>& p = ds->p;
         const Vec4<Real>* __restrict__ pos = ds->pos;
         const Vec4<Real>* __restrict__ vel = ds->vel;
-        const Real* __restrict__ rho = ds->density;  // rho - rho0
+        const Real* __restrict__ vol = ds->vol;
         const Cubic<Real> K = p.kern;
         const Vec4<Real> xi = pos[i];
         const Vec4<Real> vi = vel[i];
         const uint32_t nf = fluid_count(ds->counts[i]);
         const Real cvis = p.inv_h * p.viscosity;
         KSum3<Real> a;
-        Vec4<Real> xj[kViscBatch], vj[kViscBatch];
-        Real rj[kViscBatch];
-        visit_neighbors<kViscBatch>(
-            ds->nbr, p.nbr_stride, i, 0, nf, i,
+        Vec4<Real> xj[2], vj[2];
+        Real volj[2];
+        visit_neighbors(
+            ds->nbr + i, p.nbr_stride, nf,
             [&](int u, uint32_t j) {
                 xj[u] = ld4<Real>(pos + j);
                 vj[u] = ld4<Real>(vel + j);
-                rj[u] = p.density0 + rho[j];
+                volj[u] = __ldg(vol + j);
             },
             [&](int u) {
                 const Real w = K.W(xi.x - xj[u].x, xi.y - xj[u].y, xi.z - xj[u].z);
-                const Real sc = cvis * (xj[u].w / rj[u]);
+                const Real sc = cvis * volj[u];
                 a.add(-(sc * (vi.x - vj[u].x)) * w, -(sc * (vi.y - vj[u].y)) * w, -(sc * (vi.z - vj[u].z)) * w);
             });
         Vec4<Real> out;
@@ -728,22 +722,18 @@ __global__ void __launch_bounds__(kBlock, kGatherMinBlocks) pressure_residual_ke
                                                                    cudaGraphConditionalHandle handle,
                                                                    bool use_handle) {
     DFSPH_PDL_ENTER;
-    if (kMode == kFallback && !take_fallback(ds, 1, 2u)) return;  // uniform over the grid
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    const Vec4<Real>* __restrict__ vel = kMode == kFallback ? ds->velP : ds->vel;
+    const Vec4<Real>* __restrict__ vel = ds->vel;
     double contrib = 0.0, aux = 0.0;
     if (i < n) {
         const StepParams<Real>& p = ds->p;
-        Real alpha = ds->factor[i];  // the fallback pass finds alpha already scaled by its init pass
+        Real alpha = ds->factor[i];
         Real kap = Real(0);
         if (kMode == kInitPass) {
             alpha *= p.inv_h_future;
             ds->factor[i] = alpha;
-        } else if (kMode == kLoop) {
-            kap = ds->kappa[i];
         } else {
-            ds->vel[i] = vel[i];
-            ds->kappaW[i] = ds->kappaP[i];
+            kap = ds->kappa[i];
         }
         const Vec4<Real> xi = ds->pos[i];
         const Vec4<Real> vi = vel[i];
@@ -801,34 +791,6 @@ __global__ void __launch_bounds__(kBlock) update_pos_kernel(const DevState<Real>
     x.y += h * v.y;
     x.z += h * v.z;
     ds->pos[i] = x;
-}
-
-// Initial residual of a warm-start candidate whose velocities are `vel`, as sum |r| of the unclamped
-// residuals (probe: the sum goes to ctl[3], nothing else is written). which = 0: divergence
-// (computeDensityChange), 1: density. The solver's own criterion clamps r at 0 and so cannot see an
-// over-pressured candidate (r < 0 everywhere it pushes too hard); |r| sees both directions.
-template <class Real, int kWhich>
-__global__ void __launch_bounds__(kBlock, kGatherMinBlocks) probe_residual_kernel(const DevState<Real>* __restrict__ ds,
-                                                                              uint32_t n,
-                                                                              const Vec4<Real>* __restrict__ vel) {
-    DFSPH_PDL_ENTER;
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    double contrib = 0.0;
-    if (i < n) {
-        const StepParams<Real>& p = ds->p;
-        const uint32_t c = ds->counts[i];
-        const uint32_t nf = fluid_count(c), nb = boundary_count(c);
-        if (kWhich == 0) {
-            uint32_t num = nf;
-            if (num < kMinNeighborsForDivergence) num += nb;
-            if (num >= kMinNeighborsForDivergence)
-                contrib = fabs((double)velocity_divergence<Real>(ds, p, i, ds->pos[i], vel[i], nf, nb, vel));
-        } else {
-            const Real sdiv = velocity_divergence<Real>(ds, p, i, ds->pos[i], vel[i], nf, nb, vel);
-            contrib = fabs((double)(ds->density[i] + p.h_future * sdiv));
-        }
-    }
-    reduce_and_decide<1>(contrib, ds->partials, ds->ctl + 3, n, 0.0, 0, 1, 0, false);
 }
 
 // ---- both warm-start candidates in one pass (learned warm start with the plain fallback) ---------
@@ -1117,9 +1079,10 @@ __global__ void __launch_bounds__(kBlock) gather_training_kernel(const DevState<
 }  // namespace
 
 template <class Real>
-void launch_density_alpha(const DevState<Real>* d, uint32_t n, bool warm_v, bool features, cudaStream_t s) {
+void launch_density_alpha(const DevState<Real>* d, uint32_t n, bool warm_v, bool features, cudaStream_t s,
+                          bool rows_only) {
     if (!n) return;
-    launch_pdl(density_alpha_kernel<Real>, grid_for(n), kBlock, 0, s, d, n, warm_v && !features, features);
+    launch_pdl(density_alpha_kernel<Real>, grid_for(n), kBlock, 0, s, d, n, warm_v && !features, features, rows_only);
 }
 template <class Real>
 void launch_divergence_warm_jacobi(const DevState<Real>* d, uint32_t n, const Real* kw, Vec4<Real>* vout,
@@ -1127,12 +1090,6 @@ void launch_divergence_warm_jacobi(const DevState<Real>* d, uint32_t n, const Re
     if (!n) return;
     if (forces) launch_pdl(divergence_warm_jacobi_kernel<Real, true>, grid_for(n), kBlock, 0, s, d, n, kw, vout);
     else launch_pdl(divergence_warm_jacobi_kernel<Real, false>, grid_for(n), kBlock, 0, s, d, n, kw, vout);
-}
-template <class Real>
-void launch_probe_residual(const DevState<Real>* d, uint32_t n, int which, const Vec4<Real>* vel, cudaStream_t s) {
-    const unsigned g = grid_for(n ? n : 1);
-    if (which == 0) launch_pdl(probe_residual_kernel<Real, 0>, g, kBlock, 0, s, d, n, vel);
-    else launch_pdl(probe_residual_kernel<Real, 1>, g, kBlock, 0, s, d, n, vel);
 }
 template <class Real>
 void launch_warm_values(const DevState<Real>* d, uint32_t n, int which, bool learned, bool use_pred, double damping,
@@ -1219,15 +1176,6 @@ template <class Real> void launch_select_candidate(const DevState<Real>* d, uint
     launch_pdl(select_candidate_kernel<Real>, grid_for(n ? n : 1), kBlock, 0, s, d, n, which);
 }
 template <class Real>
-void launch_fallback_residual(const DevState<Real>* d, uint32_t n, int which, double eta, int min_it, int max_it,
-                              cudaStream_t s) {
-    const unsigned g = grid_for(n ? n : 1);
-    if (which == 0)
-        launch_pdl(divergence_residual_kernel<Real, kFallback, true>, g, kBlock, 0, s, d, n, eta, min_it, max_it, 0, false);
-    else
-        launch_pdl(pressure_residual_kernel<Real, kFallback, true>, g, kBlock, 0, s, d, n, eta, min_it, max_it, 0, false);
-}
-template <class Real>
 void launch_pressure_jacobi(const DevState<Real>* d, uint32_t n, cudaGraphConditionalHandle h, bool use_handle,
                             cudaStream_t s, bool forces) {
     if (!n) return;
@@ -1242,10 +1190,9 @@ template <class Real> void launch_cfl_reduce(const DevState<Real>* d, uint32_t n
 }
 
 #define DFSPH_INSTANTIATE_SOLVER(R)                                                                                  \
-    template void launch_density_alpha<R>(const DevState<R>*, uint32_t, bool, bool, cudaStream_t);                  \
+    template void launch_density_alpha<R>(const DevState<R>*, uint32_t, bool, bool, cudaStream_t, bool);            \
     template void launch_divergence_warm_jacobi<R>(const DevState<R>*, uint32_t, const R*, Vec4<R>*, cudaStream_t,  \
                                                    bool);                                                            \
-    template void launch_probe_residual<R>(const DevState<R>*, uint32_t, int, const Vec4<R>*, cudaStream_t);        \
     template void launch_warm_values<R>(const DevState<R>*, uint32_t, int, bool, bool, double, cudaStream_t);       \
     template void launch_totals<R>(const DevState<R>*, uint32_t, bool, cudaStream_t);                               \
     template void launch_restore_totals<R>(const DevState<R>*, uint32_t, cudaStream_t);                              \
@@ -1261,7 +1208,6 @@ template <class Real> void launch_cfl_reduce(const DevState<Real>* d, uint32_t n
                                                  cudaStream_t, bool);                                                \
     template void launch_pressure_residual<R>(const DevState<R>*, uint32_t, bool, double, int, int,                 \
                                               cudaGraphConditionalHandle, bool, cudaStream_t, bool);                 \
-    template void launch_fallback_residual<R>(const DevState<R>*, uint32_t, int, double, int, int, cudaStream_t);   \
     template void launch_warm_dual<R>(const DevState<R>*, uint32_t, int, bool, cudaStream_t, bool);                  \
     template void launch_residual_dual<R>(const DevState<R>*, uint32_t, int, double, int, int, cudaStream_t);        \
     template void launch_select_candidate<R>(const DevState<R>*, uint32_t, int, cudaStream_t);                       \

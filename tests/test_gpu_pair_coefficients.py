@@ -1,0 +1,66 @@
+"""The pair coefficients of the solver passes: list remainders (filled-up slots) against the FP64 oracle,
+and the coefficients rebuilt outside the density pass."""
+import numpy as np
+import pytest
+
+from oracle import Oracle
+from splishsplash_for_cuda_b200.dfsph import DFSPHCUDA
+from splishsplash_for_cuda_b200.scene import Configuration, Scene, box_wall, synthetic_scene
+from tests._compare import assert_field
+
+pytestmark = pytest.mark.gpu
+
+
+def _sparse_block(n, seed):
+    """n particles of a compressed, perforated lattice next to two walls of a box: list lengths from 0
+    to about 40, with and without boundary neighbours."""
+    r = 0.025
+    rng = np.random.default_rng(seed)
+    side = int(np.ceil((1.4 * n) ** (1.0 / 3.0))) + 1
+    g = np.stack(np.meshgrid(*[np.arange(side)] * 3, indexing="ij"), axis=-1).reshape(-1, 3)
+    x = (2.0 * r) + 1.8 * r * g[np.sort(rng.permutation(g.shape[0])[:n])] + rng.uniform(-0.1 * r, 0.1 * r, (n, 3))
+    cfg = Configuration(timeStepSize=0.001, particleRadius=r)
+    side_m = np.ceil((2.0 * side + 6.0)) * 2.0 * r
+    return Scene(config=cfg, fluid=x.astype(np.float32), boundary=box_wall((0, 0, 0), (side_m,) * 3, 2.0 * r).astype(np.float32),
+                 fluid_velocity=rng.uniform(-0.3, 0.3, (n, 3)).astype(np.float32))
+
+
+# Tolerances: FP64 1e-9 as in the parity tests. FP32: 2^-24 per operation, about 16 ulp per kernel
+# term, and residuals that cancel to about 1/40 of their terms over a few iterations give ~1e-4 of
+# the field's scale (a velocity below a hundredth of the largest counts against that hundredth).
+@pytest.mark.parametrize("precision,rtol", [(32, 1e-4), (64, 1e-9)])
+@pytest.mark.parametrize("n", [1, 2, 31, 33, 130, 257, 1025])
+def test_list_remainders(n, precision, rtol):
+    s = _sparse_block(n, seed=n)
+    d = DFSPHCUDA(s, precision=precision)
+    st = d.step()
+    counts = d.field("neighbor_counts").reshape(-1, 2)
+    o = Oracle(s, 64)
+    ro = o.step()
+    assert (st.iterations, st.iterations_v) == (ro["iterations"], ro["iterations_v"])
+    if n >= 130:  # every remainder of the four-slot groups occurs
+        assert set(np.unique(counts[:, 0] % 4)) == {0, 1, 2, 3} and set(np.unique(counts[:, 1] % 4)) == {0, 1, 2, 3}
+    for name, floor in (("density", 1e-3), ("factor", 1e-3), ("velocity", 1e-2), ("position", 1e-3)):
+        assert_field(name, d.field(name, np.float64), o.field(name), rtol, floor)
+
+
+@pytest.mark.parametrize("precision", [32, 64])
+def test_coefficients_rebuilt_without_a_density_pass(precision):
+    """A parameter change republishes the state, after which the pressure solve forms the coefficients
+    itself: the same bits as with the density pass's."""
+    out = []
+    for touch in (False, True):
+        s = synthetic_scene(1, counts=(11, 12, 13))
+        s.fluid_velocity = np.random.default_rng(3).uniform(-0.5, 0.5, s.fluid.shape).astype(np.float32)
+        d = DFSPHCUDA(s, precision=precision)
+        d.neighbors_search()
+        d.divergence_solve()
+        d.external_forces()
+        d.update_time_step(0.002)
+        d.update_vel()
+        if touch:
+            d.set_param("viscosity", d.get_param("viscosity"))
+        its = d.pressure_solve()
+        out.append((its, d.field("velocity", np.float64), d.field("kappa", np.float64)))
+    assert out[0][0] == out[1][0]
+    assert np.array_equal(out[0][1], out[1][1]) and np.array_equal(out[0][2], out[1][2])
