@@ -153,10 +153,13 @@ __global__ void __launch_bounds__(kBlock) validate_neighbors_kernel(uint32_t* __
 // The pass is bound by instruction issue (about 216 candidate tests per particle for ~30 accepted), so
 // a test is kept to the load, the predicate and a predicated append without a branch. Appends go to a
 // column of shared memory (ListStage) and from there to the list a whole group (four slots, 16 bytes)
-// at a time. Measured at 1 M particles with moving walls: 386 -> 347 us (250 k: 122 -> 107 us); five or
-// six blocks per SM instead of four, two or eight candidates per batch instead of four were slower by
-// 6 to 28 %.
-constexpr uint32_t kStageSlots = 24;
+// at a time. The column holds 40 entries, more than most lists, and when a lane has to flush all lanes of
+// the warp that scan with it do: with 24 entries and each lane for itself the flushes were a quarter of
+// the pass's instructions. Measured at 1 M particles, static / moving walls: 336 / 348 us -> 304 / 319 us
+// (386 us with a branch per accepted candidate and no column); 250 k 106 -> 97 us, 1 k 33 -> 29 us. Five
+// or six blocks per SM instead of four, two, five or eight candidates per batch instead of four, and two
+// particles of a cell per thread were slower or, for large scenes, at most 5 % faster.
+constexpr uint32_t kStageSlots = 40;
 constexpr uint32_t kScanBatch = 4;
 constexpr int kBuildMinBlocks = 4;
 static_assert(kScanBatch - 1 <= kScanPad, "a batch reads past the end of the last run");
@@ -209,7 +212,8 @@ template <class Real, bool kFluid>
 __device__ __forceinline__ void scan_cell(const Vec4<Real>* __restrict__ src, uint32_t j0, uint32_t j1, uint32_t i,
                                           const Vec4<Real>& xi, Real H2, ListStage& st) {
     for (uint32_t jb = j0; jb < j1; jb += kScanBatch) {
-        if (st.top > (kStageSlots - kScanBatch) * kBlock) st.flush();
+        // (a hint: which lanes scan together does not change what any of them writes)
+        if (__any_sync(__activemask(), st.top > (kStageSlots - kScanBatch) * kBlock)) st.flush();
         Vec4<Real> xj[kScanBatch];
 #pragma unroll
         for (uint32_t u = 0; u < kScanBatch; ++u) xj[u] = ld4<Real>(src + jb + u);
