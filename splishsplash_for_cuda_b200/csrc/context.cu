@@ -108,6 +108,7 @@ public:
     uint4* nbr = nullptr;
     Vec4<Real>* coef = nullptr;
     Real* vol = nullptr;
+    bool hist_zero = false;  // the sort's histograms are zero (the last fluid reorder cleared them)
     bool coef_ok = false;  // the pair coefficients match the lists and the current positions
     SortBuffers sb;
     uint2* ftab = nullptr;
@@ -429,6 +430,14 @@ public:
     }
 
     int sync_state() {
+        fill_state();
+        launch_set_state<Real>(ds, hs, stream);
+        launches += 1;
+        DF_CUDA(cudaGetLastError());
+        return DFSPH_OK;
+    }
+    // The host's copy of the state block, to be published to ds.
+    void fill_state() {
         coef_ok = false;  // the particle order, the boundary or the lists may have changed
         hs.p = params();
         hs.pos = pos[cur];
@@ -470,10 +479,6 @@ public:
         hs.out_scale = mlp.scales ? reinterpret_cast<const float*>(reinterpret_cast<const char*>(mlp.scales) +
                                                                   offsetof(MlpScales, out_scale))
                                   : nullptr;
-        launch_set_state<Real>(ds, hs, stream);
-        launches += 1;
-        DF_CUDA(cudaGetLastError());
-        return DFSPH_OK;
     }
 
     // Cell grid from a bounding box, following DFSPHCData::initGridOffset
@@ -555,14 +560,22 @@ public:
         return true;
     }
 
+    // Zeroes the sort's histograms before a key pass, unless the last fluid reorder has (a boundary sort, or
+    // a binning that returned early, leaves its counts there).
+    int zero_histograms() {
+        if (!hist_zero) DF_CUDA(cudaMemsetAsync(sort_histograms(sb), 0, kSortHistWords * sizeof(uint32_t), stream));
+        hist_zero = false;
+        return DFSPH_OK;
+    }
     // Sorts the boundary set in place by cell key and rebuilds its cell table.
     int sort_boundary(bool compute_psi) {
         const StepParams<Real> p = params();
-        launch_cell_keys<Real>(bpos[1], nb, p, sb.keys_a, status + 1, stream);
+        DF_TRY(zero_histograms());
+        launch_cell_keys<Real>(bpos[1], nb, p, sb.keys_a, status + 1, sort_histograms(sb), key_passes, stream,
+                               (uint32_t*)btab, 2 * cells, sort_clear_begin(sb), sort_clear_words(nb, key_passes));
         uint32_t *skeys, *perm;
         radix_sort_pairs(sb, nb, key_passes, true, stream, status, &launches, &skeys, &perm);
         launch_reorder_boundary<Real>(perm, nb, bpos[1], bvel[1], bpos[0], bvel[0], bid, stream);
-        DF_CUDA(cudaMemsetAsync(btab, 0, cells * sizeof(uint2), stream));
         launch_cell_bounds(skeys, nb, dim[0], dim[1], dim[2], btab, stream);
         DF_CUDA(cudaMemsetAsync(bnear, 0, cells, stream));
         launch_mark_near_boundary(skeys, nb, dim[0], dim[1], dim[2], bnear, stream);
@@ -832,24 +845,26 @@ public:
             return sync_state();
         }
         const StepParams<Real> p = params();
-        // the key pass also clears the fluid cell table and the sort's workspace (no memsets between
-        // the kernels of the step)
-        launch_cell_keys<Real>(pos[cur], n, p, sb.keys_a, status, stream, (uint32_t*)ftab, 2 * cells, sb.workspace,
-                               radix_sort_workspace_words(n, key_passes));
+        // the key pass also counts the sort's digits and clears the fluid cell table and the sort's
+        // workspace (no memsets between the kernels of the step)
+        DF_TRY(zero_histograms());
+        launch_cell_keys<Real>(pos[cur], n, p, sb.keys_a, status, sort_histograms(sb), key_passes, stream, (uint32_t*)ftab,
+                               2 * cells, sort_clear_begin(sb), sort_clear_words(n, key_passes));
         uint32_t *skeys, *perm;
-        radix_sort_pairs(sb, n, key_passes, true, stream, status, &launches, &skeys, &perm, sort_withheld_tile, true);
+        radix_sort_pairs(sb, n, key_passes, true, stream, status, &launches, &skeys, &perm, sort_withheld_tile);
         if (!defer_velocities) DF_TRY(flush_pending());  // velocities uploaded during the key pass and the sort
-        const int nx = 1 - cur;
-        launch_reorder_fluid<Real>(perm, n, pos[cur], vel[cur], kappa[cur], kappaV[cur], id[cur], pos[nx], vel[nx],
-                                   kappa[nx], kappaV[nx], id[nx], stream);
+        const int old = cur;
+        cur = 1 - cur;
         if (learned) {
-            launch_reorder_pair<Real>(perm, n, kappaT[cur], kappaVT[cur], kappaT[nx], kappaVT[nx], stream);
+            launch_reorder_pair<Real>(perm, n, kappaT[old], kappaVT[old], kappaT[cur], kappaVT[cur], stream);
             launches += 1;
         }
-        cur = nx;
-        launch_cell_bounds(skeys, n, dim[0], dim[1], dim[2], ftab, stream);
-        DF_TRY(sync_state());
-        launches += 3;
+        fill_state();
+        launch_reorder_fluid<Real>(perm, skeys, n, pos[old], vel[old], kappa[old], kappaV[old], id[old], ftab,
+                                   sort_histograms(sb), ds, hs, stream);
+        hist_zero = true;
+        launches += 2;
+        DF_CUDA(cudaGetLastError());
         return DFSPH_OK;
     }
 
@@ -2980,25 +2995,7 @@ public:
         for (int r = 0; r < reps; ++r) {
             DF_CUDA(cudaEventRecord(ev0, stream));
             if (k == DFSPH_K_SORT_REORDER) {
-                // keys -> radix sort -> reorder -> cell table: the first part of the neighbour search
-                const StepParams<Real> p = params();
-                launch_cell_keys<Real>(pos[cur], n, p, sb.keys_a, status, stream);
-                uint32_t *skeys, *perm;
-                radix_sort_pairs(sb, n, key_passes, true, stream, status, &launches, &skeys, &perm);
-                const int nx = 1 - cur;
-                launch_reorder_fluid<Real>(perm, n, pos[cur], vel[cur], kappa[cur], kappaV[cur], id[cur], pos[nx],
-                                           vel[nx], kappa[nx], kappaV[nx], id[nx], stream);
-                if (learned) {
-                    launch_reorder_pair<Real>(perm, n, kappaT[cur], kappaVT[cur], kappaT[nx], kappaVT[nx], stream);
-                    launches += 1;
-                }
-                DF_CUDA(cudaMemsetAsync(ftab, 0, cells * sizeof(uint2), stream));
-                launch_cell_bounds(skeys, n, dim[0], dim[1], dim[2], ftab, stream);
-                cur = nx;
-                launches += 3;
-                launch_set_state<Real>(ds, (hs.pos = pos[cur], hs.vel = vel[cur], hs.kappa = kappa[cur],
-                                            hs.kappaV = kappaV[cur], hs.id = id[cur], hs.kappaT = kappaT[cur],
-                                            hs.kappaVT = kappaVT[cur], hs), stream);
+                DF_TRY(bin_fluid());  // keys, sort, reorder and cell table: the first part of the neighbour search
             } else {
                 launch_kernel(k);
             }

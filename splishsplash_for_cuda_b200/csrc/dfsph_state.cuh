@@ -61,16 +61,35 @@ template <class Real> struct DevState {
 };
 
 // ---- launch wrappers (neighbors.cu) ----------------------------------------------------------------
-template <class Real>
+// The state block := v, except the dt fields, which the device keeps, and the solver loops' last-block
+// tickets, which start from zero (each reduction leaves them at zero too; resetting them here saves a
+// memset before every solve). One thread.
+template <class Real> __device__ __forceinline__ void publish_state(DevState<Real>* __restrict__ dst, DevState<Real> v) {
+    const StepParams<Real>& o = dst->p;
+    v.p.h = o.h;
+    v.p.h_future = o.h_future;
+    v.p.inv_h = o.inv_h;
+    v.p.inv_h_future = o.inv_h_future;
+    v.p.h_ratio_to_past = o.h_ratio_to_past;
+    v.p.h_ratio_to_past2 = o.h_ratio_to_past2;
+    *dst = v;
+    if (v.ctl)
+        for (int k = 0; k < 4; ++k) v.ctl[k].ticket = 0;
+}
+
+// Cell keys and the histograms of their first `passes` 8-bit digits (added to hist).
 // clear0 / clear1 (words0 / words1 32-bit words each, may be null / 0): buffers the same launch sets
-// to zero (the fluid cell table and the sort's workspace before a fluid binning).
-void launch_cell_keys(const Vec4<Real>* pos, uint32_t n, const StepParams<Real>& p, uint32_t* keys, uint32_t* status,
-                      cudaStream_t s, uint32_t* clear0 = nullptr, size_t words0 = 0, uint32_t* clear1 = nullptr,
-                      size_t words1 = 0);
+// to zero (the cell table and the sort's workspace before a binning).
 template <class Real>
-void launch_reorder_fluid(const uint32_t* perm, uint32_t n, const Vec4<Real>* pos_in, const Vec4<Real>* vel_in,
-                          const Real* kappa_in, const Real* kappaV_in, const uint32_t* id_in, Vec4<Real>* pos_out,
-                          Vec4<Real>* vel_out, Real* kappa_out, Real* kappaV_out, uint32_t* id_out, cudaStream_t s);
+void launch_cell_keys(const Vec4<Real>* pos, uint32_t n, const StepParams<Real>& p, uint32_t* keys, uint32_t* status,
+                      uint32_t* hist, int passes, cudaStream_t s, uint32_t* clear0, size_t words0, uint32_t* clear1,
+                      size_t words1);
+// Reorders the fluid into the arrays of `state`, marks the cell table, publishes `state` to *d and clears
+// the sort's histograms (kSortHistWords words).
+template <class Real>
+void launch_reorder_fluid(const uint32_t* perm, const uint32_t* sorted_keys, uint32_t n, const Vec4<Real>* pos_in,
+                          const Vec4<Real>* vel_in, const Real* kappa_in, const Real* kappaV_in, const uint32_t* id_in,
+                          uint2* table, uint32_t* hist, DevState<Real>* d, const DevState<Real>& state, cudaStream_t s);
 // Reorders two more per-particle arrays by the same permutation (learned warm-start totals).
 template <class Real>
 void launch_reorder_pair(const uint32_t* perm, uint32_t n, const Real* a_in, const Real* b_in, Real* a_out,

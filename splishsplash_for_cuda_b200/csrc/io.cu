@@ -205,18 +205,7 @@ __global__ void __launch_bounds__(kBlock) unpack_counts_kernel(const uint32_t* _
 // ordered with the surrounding work on the stream and never reads host memory asynchronously.
 template <class Real> __global__ void set_state_kernel(DevState<Real>* __restrict__ dst, DevState<Real> v) {
     DFSPH_PDL_ENTER;
-    const StepParams<Real>& o = dst->p;  // dt fields stay as the device has them
-    v.p.h = o.h;
-    v.p.h_future = o.h_future;
-    v.p.inv_h = o.inv_h;
-    v.p.inv_h_future = o.inv_h_future;
-    v.p.h_ratio_to_past = o.h_ratio_to_past;
-    v.p.h_ratio_to_past2 = o.h_ratio_to_past2;
-    *dst = v;
-    // The solver loops' last-block tickets start from zero (each reduction leaves them at zero too);
-    // resetting them here, with the state, saves a memset before every solve.
-    if (v.ctl)
-        for (int k = 0; k < 4; ++k) v.ctl[k].ticket = 0;
+    publish_state(dst, v);
 }
 
 template <class Real>

@@ -5,12 +5,13 @@
 // whose order within a cell depends on atomics. This sort is stable, so the sorted order, the
 // neighbour lists and every sum that follows are deterministic run to run.
 //
-// Design: 8-bit digits; one histogram pass computes all digit histograms; each digit pass is a
-// single "onesweep" kernel: a tile ranks its keys stably in shared memory (warp match + per-warp
-// digit counters), publishes its per-digit count, and obtains its global exclusive prefix by a
-// decoupled look-back over earlier tiles. Tiles take their index from an atomic counter at start,
-// so a tile only ever waits on tiles that are already running; every wait is bounded and gives up
-// with DFSPH_ST_SORT_TIMEOUT instead of hanging.
+// Design: 8-bit digits; all digit histograms are counted before the first pass (by the pass that
+// forms the keys); each digit pass is a single "onesweep" kernel: a tile scans its pass's histogram,
+// ranks its keys stably in shared memory (warp match + per-warp digit counters), publishes its
+// per-digit count, and obtains its global exclusive prefix by a decoupled look-back over earlier
+// tiles. Tiles take their index from an atomic counter at start, so a tile only ever waits on tiles
+// that are already running; every wait is bounded and gives up with DFSPH_ST_SORT_TIMEOUT instead of
+// hanging.
 #include <string>
 
 #include "dfsph_common.cuh"
@@ -47,44 +48,38 @@ __global__ void __launch_bounds__(kSortThreads) histogram_kernel(const uint32_t*
     }
 }
 
-// Exclusive scan of each pass's 256-bin histogram (one block of 256 threads).
-__global__ void __launch_bounds__(256) scan_kernel(const uint32_t* __restrict__ hist, int passes,
-                                                   uint32_t* __restrict__ offsets) {
-    DFSPH_PDL_ENTER;
-    __shared__ uint32_t s[256];
-    for (int p = 0; p < passes; ++p) {
-        const uint32_t v = hist[p * 256 + threadIdx.x];
-        s[threadIdx.x] = v;
-        __syncthreads();
-        for (int d = 1; d < 256; d <<= 1) {
-            const uint32_t add = threadIdx.x >= d ? s[threadIdx.x - d] : 0u;
-            __syncthreads();
-            s[threadIdx.x] += add;
-            __syncthreads();
-        }
-        offsets[p * 256 + threadIdx.x] = s[threadIdx.x] - v;
-        __syncthreads();
-    }
-}
-
 __device__ __forceinline__ uint32_t ld_volatile(const uint32_t* p) { return *(const volatile uint32_t*)p; }
 __device__ __forceinline__ void st_volatile(uint32_t* p, uint32_t v) { *(volatile uint32_t*)p = v; }
 
 __global__ void __launch_bounds__(kSortThreads) onesweep_kernel(
     const uint32_t* __restrict__ kin, const uint32_t* __restrict__ vin, uint32_t* __restrict__ kout,
-    uint32_t* __restrict__ vout, uint32_t n, int shift, uint32_t key_mask, const uint32_t* __restrict__ digit_offsets,
+    uint32_t* __restrict__ vout, uint32_t n, int shift, uint32_t key_mask, const uint32_t* __restrict__ hist,
     uint32_t* __restrict__ tile_status, uint32_t* __restrict__ tile_counter, uint32_t* __restrict__ status_word,
     uint32_t withheld_tile) {
     DFSPH_PDL_ENTER;
     __shared__ uint32_t warp_hist[kSortWarps][256];
     __shared__ uint32_t digit_base[256];
     __shared__ uint32_t s_tile;
+    __shared__ uint32_t digit_warp_total[kSortWarps];
 
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
     for (int t = threadIdx.x; t < kSortWarps * 256; t += kSortThreads) (&warp_hist[0][0])[t] = 0;
     if (threadIdx.x == 0) s_tile = atomicAdd(tile_counter, 1u);
+    // Exclusive scan of the pass's histogram, one digit per thread (every tile does it for itself, which
+    // costs less than a launch between the histograms and the first pass): within the warp here, the
+    // preceding warps' totals below.
+    const uint32_t digit_count = hist[threadIdx.x];
+    uint32_t digit_offset = digit_count;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t v = __shfl_up_sync(0xFFFFFFFFu, digit_offset, o);
+        if (lane >= o) digit_offset += v;
+    }
+    if (lane == 31) digit_warp_total[warp] = digit_offset;
+    digit_offset -= digit_count;
     __syncthreads();
+    for (int w = 0; w < warp; ++w) digit_offset += digit_warp_total[w];
     const uint32_t tile = s_tile;
     const uint32_t base = tile * kSortTile + warp * (kSortItems * 32);
 
@@ -144,7 +139,7 @@ __global__ void __launch_bounds__(kSortThreads) onesweep_kernel(
             }
             if (publish) st_volatile(my, kFlagPrefix | ((exclusive + total) & kCountMask));
         }
-        digit_base[d] = digit_offsets[d] + exclusive;
+        digit_base[d] = digit_offset + exclusive;
     }
     __syncthreads();
 
@@ -165,7 +160,7 @@ __global__ void __launch_bounds__(kSortThreads) onesweep_kernel(
 
 size_t radix_sort_workspace_words(uint32_t n_max, int passes) {
     const size_t tiles = (n_max + kSortTile - 1) / kSortTile;
-    return 4 + 1024 + 1024 + (size_t)passes * tiles * 256;
+    return kSortHistWords + 4 + (size_t)passes * tiles * kSortDigits;
 }
 
 // Sorts (keys_a, vals_a) by key. Pass p reads buffer set (p even ? a : b) and writes the other;
@@ -173,26 +168,17 @@ size_t radix_sort_workspace_words(uint32_t n_max, int passes) {
 // *keys_out / *vals_out and lies in set a after an even number of passes, else in set b.
 void radix_sort_pairs(SortBuffers& b, uint32_t n, int passes, bool iota_values, cudaStream_t stream,
                       uint32_t* status_word, uint64_t* launch_counter, uint32_t** keys_out, uint32_t** vals_out,
-                      uint32_t withheld_tile, bool workspace_cleared) {
+                      uint32_t withheld_tile) {
     if (n == 0 || passes == 0) {
         *keys_out = b.keys_a;
         *vals_out = b.vals_a;
         return;
     }
     const size_t tiles = (n + kSortTile - 1) / kSortTile;
-    // workspace: [0,4) tile counters, [4,1028) histograms, [1028,2052) digit offsets, then tile status
-    uint32_t* counters = b.workspace;
-    uint32_t* hist = b.workspace + 4;
-    uint32_t* offsets = hist + 1024;
-    uint32_t* status = offsets + 1024;
-    if (!workspace_cleared)
-        cudaMemsetAsync(b.workspace, 0, radix_sort_workspace_words(n, passes) * sizeof(uint32_t), stream);
-    int hist_blocks = (int)((n + kSortThreads * 16 - 1) / (kSortThreads * 16));
-    if (hist_blocks > 148 * 4) hist_blocks = 148 * 4;
-    if (hist_blocks < 1) hist_blocks = 1;
-    launch_pdl(histogram_kernel, hist_blocks, kSortThreads, 0, stream, b.keys_a, n, passes, 0xFFFFFFFFu, hist);
-    launch_pdl(scan_kernel, 1, 256, 0, stream, hist, passes, offsets);
-    *launch_counter += 2;
+    // workspace: the histograms, the tile counters of the passes, then the tile status
+    const uint32_t* hist = sort_histograms(b);
+    uint32_t* counters = sort_clear_begin(b);
+    uint32_t* status = counters + 4;
     for (int p = 0; p < passes; ++p) {
         const bool even = (p & 1) == 0;
         const uint32_t* kin = even ? b.keys_a : b.keys_b;
@@ -200,9 +186,8 @@ void radix_sort_pairs(SortBuffers& b, uint32_t n, int passes, bool iota_values, 
         uint32_t* kout = even ? b.keys_b : b.keys_a;
         uint32_t* vout = even ? b.vals_b : b.vals_a;
         launch_pdl(onesweep_kernel, (unsigned)tiles, kSortThreads, 0, stream, kin, vin, kout, vout, n, 8 * p, 0xFFFFFFFFu,
-                   offsets + p * 256,
-                                                                   status + (size_t)p * tiles * 256, counters + p,
-                                                                   status_word, withheld_tile);
+                   hist + p * kSortDigits, status + (size_t)p * tiles * kSortDigits, counters + p, status_word,
+                   withheld_tile);
         *launch_counter += 1;
     }
     const bool in_a = (passes & 1) == 0;
@@ -223,11 +208,11 @@ void radix_sort_pairs(SortBuffers& b, uint32_t n, int passes, bool iota_values, 
 namespace {
 constexpr uint32_t kNoAllocMaxKeys = 1u << 18;  // 262,144 keys per call
 constexpr size_t kNoAllocTiles = (kNoAllocMaxKeys + kSortTile - 1) / kSortTile;
-// layout (32-bit words): [0,4) tile counters, [4,8) status word, [8,1032) digit histograms,
-// [1032,2056) digit offsets, then 4 passes of tile look-back flags, then the ping-pong keys and
-// payloads. Everything before the ping-pong pair is cleared at the start of every call.
-constexpr size_t kNoAllocCounters = 0, kNoAllocStatus = 4, kNoAllocHist = 8, kNoAllocOffsets = 1032;
-constexpr size_t kNoAllocTileFlags = 2056;
+// layout (32-bit words): [0,4) tile counters, [4,8) status word, [8,1032) digit histograms, then 4
+// passes of tile look-back flags, then the ping-pong keys and payloads. Everything before the
+// ping-pong pair is cleared at the start of every call.
+constexpr size_t kNoAllocCounters = 0, kNoAllocStatus = 4, kNoAllocHist = 8;
+constexpr size_t kNoAllocTileFlags = 1032;
 constexpr size_t kNoAllocClearWords = kNoAllocTileFlags + 4 * kNoAllocTiles * 256;
 constexpr size_t kNoAllocWords = kNoAllocClearWords + 2 * (size_t)kNoAllocMaxKeys;
 static __device__ __align__(256) uint32_t g_noalloc_scratch[kNoAllocWords];
@@ -277,7 +262,6 @@ extern "C" int dfsph_sort_cell_keys_noalloc(const uint32_t* keys_in, uint32_t* k
     uint32_t* counters = scratch + kNoAllocCounters;
     uint32_t* status = scratch + kNoAllocStatus;
     uint32_t* hist = scratch + kNoAllocHist;
-    uint32_t* offsets = scratch + kNoAllocOffsets;
     uint32_t* flags = scratch + kNoAllocTileFlags;
     uint32_t* pk = scratch + kNoAllocClearWords;  // ping-pong keys
     uint32_t* pv = pk + kNoAllocMaxKeys;           // ping-pong payloads
@@ -286,7 +270,6 @@ extern "C" int dfsph_sort_cell_keys_noalloc(const uint32_t* keys_in, uint32_t* k
     int hist_blocks = (int)((n + kSortThreads * 16 - 1) / (kSortThreads * 16));
     if (hist_blocks > 148 * 4) hist_blocks = 148 * 4;
     launch_pdl(histogram_kernel, hist_blocks, kSortThreads, 0, s, keys_in, n, passes, key_mask, hist);
-    launch_pdl(scan_kernel, 1, 256, 0, s, hist, passes, offsets);
     // The last pass must write the caller's buffers: with an odd pass count the first pass writes
     // them, with an even count the first pass writes the scratch pair.
     const uint32_t* kin = keys_in;
@@ -296,7 +279,7 @@ extern "C" int dfsph_sort_cell_keys_noalloc(const uint32_t* keys_in, uint32_t* k
         uint32_t* kout = to_out ? keys_out : pk;
         uint32_t* vout = to_out ? perm_out : pv;
         launch_pdl(onesweep_kernel, (unsigned)tiles, kSortThreads, 0, s, kin, vin, kout, vout, n, 8 * p, key_mask,
-                   offsets + p * 256, flags + (size_t)p * tiles * 256, counters + p, status, kNoWithheldTile);
+                   hist + p * kSortDigits, flags + (size_t)p * tiles * 256, counters + p, status, kNoWithheldTile);
         kin = kout;
         vin = vout;
         to_out = !to_out;
