@@ -133,7 +133,15 @@ public:
     float* cfl_partials = nullptr;
     float* stage = nullptr;      // upload staging: 7 floats per particle of max(Nc, Bc)
     void* dl = nullptr;          // download staging: 3 doubles per particle of max(Nc, Bc)
-    LoopCtl* h_ctl = nullptr;    // pinned mirror of ctl[0..2]
+    // What a step reads back, side by side (one copy): the loop control blocks, the dt history and the
+    // status words; ctl, dtd and status point into it, h_ctl, h_dt and h_status into its pinned mirror.
+    struct Readback {
+        LoopCtl ctl[4];
+        double dt[kDtSlots];
+        uint32_t status[4];
+    };
+    Readback *readback = nullptr, *h_readback = nullptr;
+    LoopCtl* h_ctl = nullptr;
     uint32_t* h_status = nullptr;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     bool timing = false;
@@ -294,15 +302,17 @@ public:
         DF_TRY(dalloc(&sb.workspace, radix_sort_workspace_words(nmax, 4)));
         DF_TRY(dalloc(&partials, 4 * ((size_t)grid_for(nmax) + 1)));  // two pairs of sums per block at most
         DF_TRY(dalloc(&cfl_partials, grid_for(nmax) + 1));
-        DF_TRY(dalloc(&ctl, 4));
-        DF_TRY(dalloc(&status, 4));
         DF_TRY(dalloc(&stage, (size_t)nmax * 7));
         DF_CUDA(cudaMalloc(&dl, (size_t)nmax * 3 * sizeof(double)));
         DF_CUDA(cudaMalloc((void**)&ds, sizeof(DevState<Real>)));
-        DF_CUDA(cudaMallocHost((void**)&h_ctl, 3 * sizeof(LoopCtl)));
-        DF_CUDA(cudaMallocHost((void**)&h_status, 4 * sizeof(uint32_t)));
-        DF_TRY(dalloc(&dtd, kDtSlots));
-        DF_CUDA(cudaMallocHost((void**)&h_dt, kDtSlots * sizeof(double)));
+        DF_TRY(dalloc(&readback, 1));
+        ctl = readback->ctl;
+        dtd = readback->dt;
+        status = readback->status;
+        DF_CUDA(cudaMallocHost((void**)&h_readback, sizeof(Readback)));
+        h_ctl = h_readback->ctl;
+        h_dt = h_readback->dt;
+        h_status = h_readback->status;
         DF_CUDA(cudaMemsetAsync(ctl, 0, 4 * sizeof(LoopCtl), stream));
         DF_CUDA(cudaMemsetAsync(status, 0, 4 * sizeof(uint32_t), stream));
         DF_CUDA(cudaMemsetAsync(counts, 0, Nc * sizeof(uint32_t), stream));
@@ -331,7 +341,7 @@ public:
         }
         f(density); f(factor); f(densityAdv); f(kcoef); f(acc); f(counts); f(nbr); f(coef); f(vol); f(bid); f(bforce); f(bforce_fx);
         f(sb.keys_a); f(sb.keys_b); f(sb.vals_a); f(sb.vals_b); f(sb.workspace);
-        f(partials); f(cfl_partials); f(ctl); f(status); f(stage); f(dl); f(ds); f(ftab); f(btab); f(bnear);
+        f(partials); f(cfl_partials); f(readback); f(stage); f(dl); f(ds); f(ftab); f(btab); f(bnear);
         for (int b = 0; b < 2; ++b) {
             f(kappaT[b]); f(kappaVT[b]);
         }
@@ -347,11 +357,8 @@ public:
             m = MeshSlot{};
         }
         if (h_ob) cudaFreeHost(h_ob);
-        if (h_ctl) cudaFreeHost(h_ctl);
-        if (h_status) cudaFreeHost(h_status);
-        if (h_dt) cudaFreeHost(h_dt);
+        if (h_readback) cudaFreeHost(h_readback);
         if (h_loss) cudaFreeHost(h_loss);
-        f(dtd);
         if (ev0) cudaEventDestroy(ev0);
         if (ev1) cudaEventDestroy(ev1);
         if (stream) cudaStreamDestroy(stream);
@@ -1799,14 +1806,13 @@ public:
     // cuda_CFL (DFSPH_core_cuda.cu:3321-3394): dt = cfl * 0.4 * 2r / sqrt(max |v + a h|^2), clamped,
     // reduced and applied on the device (no host round trip).
     int cfl(double min_dt, double factor_, double max_dt) {
-        launch_cfl_reduce<Real>(ds, n ? grid_for(n) : 0, stream);
         DtArgs a{};
         a.v[0] = factor_;
         a.v[1] = min_dt;
         a.v[2] = max_dt;
         a.v[3] = 2.0 * sc.particle_radius;
-        launch_dt<Real>(ds, 2, a, stream);
-        launches += 2;
+        launch_cfl<Real>(ds, n ? grid_for(n) : 0, a, stream);
+        launches += 1;
         dt_stale = true;
         DF_CUDA(cudaGetLastError());
         return DFSPH_OK;
@@ -1821,9 +1827,10 @@ public:
         return DFSPH_OK;
     }
 
-    int update_pos() {
+    int update_pos(const EscapeBox& box = {}, bool end_step = false) {
         if (!n) return DFSPH_OK;
-        launch_update_pos<Real>(ds, n, stream);
+        launch_update_pos<Real>(ds, n, stream, box, end_step);
+        if (end_step) dt_stale = true;
         coef_ok = false;
         launches += 1;
         DF_CUDA(cudaGetLastError());
@@ -1840,9 +1847,7 @@ public:
 
     // Reads the loop control blocks and the status word (one synchronisation).
     int collect(bool div_ran, int max_iter_v, int max_iter) {
-        DF_CUDA(cudaMemcpyAsync(h_ctl, ctl, 2 * sizeof(LoopCtl), cudaMemcpyDeviceToHost, stream));
-        DF_CUDA(cudaMemcpyAsync(h_status, status, 4 * sizeof(uint32_t), cudaMemcpyDeviceToHost, stream));
-        DF_CUDA(cudaMemcpyAsync(h_dt, dtd, kDtSlots * sizeof(double), cudaMemcpyDeviceToHost, stream));
+        DF_CUDA(cudaMemcpyAsync(h_readback, readback, sizeof(Readback), cudaMemcpyDeviceToHost, stream));
         DF_CUDA(cudaStreamSynchronize(stream));
         mirror_dt();
         last_iters = n ? h_ctl[1].iter : 0;
@@ -1942,7 +1947,16 @@ public:
             DF_TRY(update_time_step(time_step));
         }
         DF_TRY(pressure_solve(sc.max_iterations, sc.max_error, true, lp));
-        DF_TRY(update_pos());
+        // DFSPHCUDA::step ends with checkParticlesPositions(2) (DFSPH_CUDA.cpp:456): the count comes
+        // back with the status words; the removal itself runs only when there is something to remove.
+        const bool tag = st && remove_escaped && n > 0;
+        EscapeBox box{};
+        if (tag) {
+            DF_TRY(ensure_scan_scratch());
+            box = EscapeBox{{bb_lo[0], bb_lo[1], bb_lo[2]}, {bb_hi[0], bb_hi[1], bb_hi[2]}, sb.keys_a, status + 3};
+        }
+        const bool end = n > 0 && !lp;  // a learned step trains on the dt of its solves first
+        DF_TRY(update_pos(box, end));
         if (lp) {
             const bool due = train_interval > 0 &&
                              (lsteps == (uint64_t)train_start ||
@@ -1952,18 +1966,9 @@ public:
             launches += 1;
             ++lsteps;
         }
-        DF_TRY(on_step_end());
+        if (!end) DF_TRY(on_step_end());
         if (timing) DF_CUDA(cudaEventRecord(ev1, stream));
         if (!st) return DFSPH_OK;  // asynchronous step: nothing read back, the host does not wait
-        // DFSPHCUDA::step ends with checkParticlesPositions(2) (DFSPH_CUDA.cpp:456): the count comes
-        // back with the status words; the removal itself runs only when there is something to remove.
-        const bool tag = remove_escaped && n > 0;
-        if (tag) {
-            DF_TRY(ensure_scan_scratch());
-            DF_CUDA(cudaMemsetAsync(status + 3, 0, sizeof(uint32_t), stream));
-            launch_box_tag<Real>(pos[cur], n, bb_lo, bb_hi, sb.keys_a, status + 3, stream);
-            launches += 1;
-        }
         DF_TRY(collect(div, sc.max_iterations_v, sc.max_iterations));
         if (tag && h_status[3]) DF_TRY(remove_tagged(h_status[3]));
         if (lp) {
@@ -2387,12 +2392,11 @@ public:
         if (!n) return DFSPH_OK;
         float* px = (float*)dl;
         float* pv = px + 3 * (size_t)n;
-        if (xyz) launch_pack_field<Real, float>((const Real*)pos[cur], 4, 3, id[cur], n, px, stream);
-        if (vxyz) launch_pack_field<Real, float>((const Real*)vel[cur], 4, 3, id[cur], n, pv, stream);
+        launch_pack_dynamic<Real>(pos[cur], vel[cur], id[cur], n, xyz ? px : nullptr, vxyz ? pv : nullptr, stream);
         if (xyz) DF_CUDA(cudaMemcpyAsync(xyz, px, 3 * (size_t)n * sizeof(float), cudaMemcpyDeviceToHost, stream));
         if (vxyz) DF_CUDA(cudaMemcpyAsync(vxyz, pv, 3 * (size_t)n * sizeof(float), cudaMemcpyDeviceToHost, stream));
         DF_CUDA(cudaStreamSynchronize(stream));
-        launches += (xyz ? 1 : 0) + (vxyz ? 1 : 0);
+        launches += 1;
         return DFSPH_OK;
     }
 

@@ -40,7 +40,8 @@ template <class Real> struct DevState {
     double* partials;      // one FP64 partial per block
     LoopCtl* ctl;          // [0] divergence loop, [1] pressure loop, [2] CFL / misc, [3] plain warm-start candidate
     double* dtd;           // dt history in FP64 (see DtSlot); the kernels read their Real copies in p
-    uint32_t* status;      // [0] DFSPH_ST_* bits, [1] scratch, [2] learned warm start kept (bit 0 div, 1 pressure)
+    uint32_t* status;      // [0] DFSPH_ST_* bits, [1] scratch, [2] learned warm start kept (bit 0 div, 1 pressure),
+                           // [3] particles outside the domain box
     float* cfl_partials;   // per-block max |v + a h|^2
     // learned warm start (see mlp.cuh)
     float* features;       // kMlpIn per particle, written by the density+alpha pass
@@ -63,7 +64,7 @@ template <class Real> struct DevState {
 // ---- launch wrappers (neighbors.cu) ----------------------------------------------------------------
 // The state block := v, except the dt fields, which the device keeps, and the solver loops' last-block
 // tickets, which start from zero (each reduction leaves them at zero too; resetting them here saves a
-// memset before every solve). One thread.
+// memset before every solve), and the count of escaped particles. One thread.
 template <class Real> __device__ __forceinline__ void publish_state(DevState<Real>* __restrict__ dst, DevState<Real> v) {
     const StepParams<Real>& o = dst->p;
     v.p.h = o.h;
@@ -75,6 +76,7 @@ template <class Real> __device__ __forceinline__ void publish_state(DevState<Rea
     *dst = v;
     if (v.ctl)
         for (int k = 0; k < 4; ++k) v.ctl[k].ticket = 0;
+    if (v.status) v.status[3] = 0;
 }
 
 // Cell keys and the histograms of their first `passes` 8-bit digits (added to hist).
@@ -178,8 +180,20 @@ template <class Real> void launch_select_candidate(const DevState<Real>* d, uint
 template <class Real>
 void launch_pressure_jacobi(const DevState<Real>* d, uint32_t n, cudaGraphConditionalHandle h, bool use_handle,
                             cudaStream_t s, bool forces = false);
-template <class Real> void launch_update_pos(const DevState<Real>* d, uint32_t n, cudaStream_t s);
-template <class Real> void launch_cfl_reduce(const DevState<Real>* d, uint32_t n_blocks, cudaStream_t s);
+// A box, and where to flag (1 inside, 0 outside) and count the particles outside it (alive null: nowhere).
+struct EscapeBox {
+    float lo[3], hi[3];
+    uint32_t* alive;
+    uint32_t* count;  // zero before the launch
+};
+// A coordinate above the box maximum or below its minimum (NaN coordinates compare false: not outside).
+template <class Real> __device__ __forceinline__ bool outside_box(const Vec4<Real>& x, const EscapeBox& b) {
+    return x.x > (Real)b.hi[0] || x.y > (Real)b.hi[1] || x.z > (Real)b.hi[2] || x.x < (Real)b.lo[0] ||
+           x.y < (Real)b.lo[1] || x.z < (Real)b.lo[2];
+}
+// end_step: also advances the dt history (advance_dt op 3).
+template <class Real>
+void launch_update_pos(DevState<Real>* d, uint32_t n, cudaStream_t s, const EscapeBox& box = {}, bool end_step = false);
 
 inline unsigned grid_for(uint32_t n) { return (n + kBlock - 1) / kBlock; }
 

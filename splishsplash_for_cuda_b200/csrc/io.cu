@@ -180,6 +180,30 @@ __global__ void __launch_bounds__(kBlock) pack_field_kernel(const Real* __restri
     for (int c = 0; c < comps; ++c) dst[(size_t)t * comps + c] = (Out)src[(size_t)i * src_stride + c];
 }
 
+// Positions and velocities (either may be null) in id order, in one pass over the ids.
+template <class Real>
+__global__ void __launch_bounds__(kBlock) pack_dynamic_kernel(const Vec4<Real>* __restrict__ pos,
+                                                              const Vec4<Real>* __restrict__ vel,
+                                                              const uint32_t* __restrict__ id, uint32_t n,
+                                                              float* __restrict__ xyz, float* __restrict__ vxyz) {
+    DFSPH_PDL_ENTER;
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const size_t t = 3 * (size_t)id[i];
+    if (xyz) {
+        const Vec4<Real> x = pos[i];
+        xyz[t] = (float)x.x;
+        xyz[t + 1] = (float)x.y;
+        xyz[t + 2] = (float)x.z;
+    }
+    if (vxyz) {
+        const Vec4<Real> v = vel[i];
+        vxyz[t] = (float)v.x;
+        vxyz[t + 1] = (float)v.y;
+        vxyz[t + 2] = (float)v.z;
+    }
+}
+
 __global__ void __launch_bounds__(kBlock) pack_u32_kernel(const uint32_t* __restrict__ src, int comps,
                                                           const uint32_t* __restrict__ id, uint32_t n,
                                                           uint32_t* __restrict__ dst) {
@@ -254,36 +278,7 @@ __global__ void __launch_bounds__(kBlock) damp_tagged_kernel(Vec4<Real>* __restr
 
 template <class Real> __global__ void dt_kernel(DevState<Real>* __restrict__ ds, int op, DtArgs a) {
     DFSPH_PDL_ENTER;
-    double* t = ds->dtd;
-    StepParams<Real>& p = ds->p;
-    if (op == 0) {
-        for (int k = 0; k < kDtSlots; ++k) t[k] = a.v[k];
-    } else if (op == 1 || op == 2) {
-        double hf;
-        if (op == 1) {
-            hf = a.v[0] > 0.0 ? a.v[0] : t[kDtFixed];
-        } else {
-            const double vmax2 = ds->ctl[2].sum;
-            hf = a.v[0] * 0.4 * (a.v[3] / sqrt(vmax2));
-            hf = (a.v[2] < hf) ? a.v[2] : hf;  // std::min(hf, max), NaN as std::min treats it
-            hf = (hf < a.v[1]) ? a.v[1] : hf;  // std::max(hf, min)
-        }
-        const double h = t[kDtH];
-        t[kDtHFuture] = hf;
-        t[kDtInvHFuture] = 1.0 / hf;
-        t[kDtRatio] = h / hf;
-        t[kDtRatio2] = (h * h) / (hf * hf);
-    } else {  // op 3
-        t[kDtHPast] = t[kDtH];
-        t[kDtH] = t[kDtHFuture];
-        t[kDtInvH] = t[kDtInvHFuture];
-    }
-    p.h = (Real)t[kDtH];
-    p.h_future = (Real)t[kDtHFuture];
-    p.inv_h = (Real)t[kDtInvH];
-    p.inv_h_future = (Real)t[kDtInvHFuture];
-    p.h_ratio_to_past = (Real)t[kDtRatio];
-    p.h_ratio_to_past2 = (Real)t[kDtRatio2];
+    advance_dt(ds, op, a);
 }
 
 }  // namespace
@@ -353,6 +348,11 @@ void launch_pack_field(const Real* src, int src_stride, int comps, const uint32_
                        cudaStream_t s) {
     if (n) launch_pdl(pack_field_kernel<Real, Out>, grid_for(n), kBlock, 0, s, src, src_stride, comps, id, n, dst);
 }
+template <class Real>
+void launch_pack_dynamic(const Vec4<Real>* pos, const Vec4<Real>* vel, const uint32_t* id, uint32_t n, float* xyz,
+                         float* vxyz, cudaStream_t s) {
+    if (n) launch_pdl(pack_dynamic_kernel<Real>, grid_for(n), kBlock, 0, s, pos, vel, id, n, xyz, vxyz);
+}
 void launch_pack_u32(const uint32_t* src, int comps, const uint32_t* id, uint32_t n, uint32_t* dst, cudaStream_t s) {
     if (n) launch_pdl(pack_u32_kernel, grid_for(n), kBlock, 0, s, src, comps, id, n, dst);
 }
@@ -380,6 +380,8 @@ void launch_unpack_counts(const uint32_t* counts, const uint32_t* id, uint32_t n
     template void launch_restore_untagged<R>(Vec4<R>*, Vec4<R>*, const uint32_t*, uint32_t, uint32_t,                \
                                              const Vec4<R>*, const Vec4<R>*, cudaStream_t);                          \
     template void launch_damp_tagged<R>(Vec4<R>*, const uint32_t*, uint32_t, uint32_t, R, cudaStream_t);             \
+    template void launch_pack_dynamic<R>(const Vec4<R>*, const Vec4<R>*, const uint32_t*, uint32_t, float*, float*,    \
+                                         cudaStream_t);                                                              \
     template void launch_pack_field<R, float>(const R*, int, int, const uint32_t*, uint32_t, float*, cudaStream_t);  \
     template void launch_pack_field<R, double>(const R*, int, int, const uint32_t*, uint32_t, double*, cudaStream_t);
 

@@ -5,7 +5,7 @@
 namespace dfsph {
 
 // Publishes the host's DevState block. The dt fields of p are kept from the device: the dt history
-// lives on the device (DtSlot) and only launch_dt changes it.
+// lives on the device (DtSlot) and only advance_dt changes it.
 template <class Real> void launch_set_state(DevState<Real>* dst, const DevState<Real>& v, cudaStream_t s);
 
 // Slots of the FP64 dt block (DevState::dtd).
@@ -19,6 +19,41 @@ struct DtArgs {
 // from ctl[2].sum, clamped to [min, max] (a.v = factor, min, max, diameter); op 3: onSimulationStepEnd.
 // Ops 1 and 2 then set 1/h_future and the ratios (DFSPHCData::updateTimeStep,
 // DFSPH_c_arrays_structure.cpp:1100-1112), all in FP64, and refresh the Real copies in p.
+template <class Real> __device__ __forceinline__ void advance_dt(DevState<Real>* __restrict__ ds, int op, const DtArgs& a) {
+    double* t = ds->dtd;
+    StepParams<Real>& p = ds->p;
+    if (op == 0) {
+        for (int k = 0; k < kDtSlots; ++k) t[k] = a.v[k];
+    } else if (op == 1 || op == 2) {
+        double hf;
+        if (op == 1) {
+            hf = a.v[0] > 0.0 ? a.v[0] : t[kDtFixed];
+        } else {
+            const double vmax2 = ds->ctl[2].sum;
+            hf = a.v[0] * 0.4 * (a.v[3] / sqrt(vmax2));
+            hf = (a.v[2] < hf) ? a.v[2] : hf;  // std::min(hf, max), NaN as std::min treats it
+            hf = (hf < a.v[1]) ? a.v[1] : hf;  // std::max(hf, min)
+        }
+        const double h = t[kDtH];
+        t[kDtHFuture] = hf;
+        t[kDtInvHFuture] = 1.0 / hf;
+        t[kDtRatio] = h / hf;
+        t[kDtRatio2] = (h * h) / (hf * hf);
+    } else {  // op 3
+        t[kDtHPast] = t[kDtH];
+        t[kDtH] = t[kDtHFuture];
+        t[kDtInvH] = t[kDtInvHFuture];
+    }
+    p.h = (Real)t[kDtH];
+    p.h_future = (Real)t[kDtHFuture];
+    p.inv_h = (Real)t[kDtInvH];
+    p.inv_h_future = (Real)t[kDtInvHFuture];
+    p.h_ratio_to_past = (Real)t[kDtRatio];
+    p.h_ratio_to_past2 = (Real)t[kDtRatio2];
+}
+// cuda_CFL: the maximum of the viscosity pass's n_blocks partials, then advance_dt op 2 with a (solver.cu).
+template <class Real> void launch_cfl(DevState<Real>* d, uint32_t n_blocks, const DtArgs& a, cudaStream_t s);
+// advance_dt in a launch of its own.
 template <class Real> void launch_dt(DevState<Real>* d, int op, const DtArgs& a, cudaStream_t s);
 
 // Writes n particles (positions, optional velocities and masses; kappa and kappa_v zero) at pos..,
@@ -64,6 +99,9 @@ void launch_restore_untagged(Vec4<Real>* pos, Vec4<Real>* vel, const uint32_t* i
                              const Vec4<Real>* spos, const Vec4<Real>* svel, cudaStream_t s);
 template <class Real>
 void launch_damp_tagged(Vec4<Real>* vel, const uint32_t* id, uint32_t n, uint32_t first, Real f, cudaStream_t s);
+template <class Real>
+void launch_pack_dynamic(const Vec4<Real>* pos, const Vec4<Real>* vel, const uint32_t* id, uint32_t n, float* xyz,
+                         float* vxyz, cudaStream_t s);
 template <class Real, class Out>
 void launch_pack_field(const Real* src, int src_stride, int comps, const uint32_t* id, uint32_t n, Out* dst,
                        cudaStream_t s);

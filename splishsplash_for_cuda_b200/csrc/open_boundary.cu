@@ -465,17 +465,13 @@ __global__ void __launch_bounds__(kBlock) compact_fluid_kernel(
 // checkParticlesPositions(2) (SPH_other_systems_cuda.cu:1242-1281): a particle with any coordinate
 // above the box maximum or below its minimum is removed (NaN coordinates compare false and stay).
 template <class Real>
-__global__ void __launch_bounds__(kBlock) box_tag_kernel(const Vec4<Real>* __restrict__ pos, uint32_t n, float lo_x,
-                                                         float lo_y, float lo_z, float hi_x, float hi_y, float hi_z,
-                                                         uint32_t* __restrict__ alive, uint32_t* __restrict__ count) {
+__global__ void __launch_bounds__(kBlock) box_tag_kernel(const Vec4<Real>* __restrict__ pos, uint32_t n, EscapeBox box) {
     DFSPH_PDL_ENTER;
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    const Vec4<Real> x = pos[i];
-    const bool out = x.x > (Real)hi_x || x.y > (Real)hi_y || x.z > (Real)hi_z || x.x < (Real)lo_x ||
-                     x.y < (Real)lo_y || x.z < (Real)lo_z;
-    alive[i] = out ? 0u : 1u;
-    if (out) atomicAdd(count, 1u);
+    const bool out = outside_box<Real>(pos[i], box);
+    box.alive[i] = out ? 0u : 1u;
+    if (out) atomicAdd(box.count, 1u);
 }
 
 __global__ void __launch_bounds__(kBlock) alive_by_id_kernel(const uint32_t* __restrict__ id,
@@ -570,8 +566,8 @@ template <class Real>
 void launch_box_tag(const Vec4<Real>* pos, uint32_t n, const float lo[3], const float hi[3], uint32_t* alive,
                     uint32_t* count, cudaStream_t s) {
     if (n)
-        launch_pdl(box_tag_kernel<Real>, grid_for(n), kBlock, 0, s, pos, n, lo[0], lo[1], lo[2], hi[0], hi[1], hi[2], alive,
-                                                            count);
+        launch_pdl(box_tag_kernel<Real>, grid_for(n), kBlock, 0, s, pos, n,
+                   EscapeBox{{lo[0], lo[1], lo[2]}, {hi[0], hi[1], hi[2]}, alive, count});
 }
 void launch_alive_by_id(const uint32_t* id, const uint32_t* alive, uint32_t n, uint32_t* alive_by_id, cudaStream_t s) {
     if (n) launch_pdl(alive_by_id_kernel, grid_for(n), kBlock, 0, s, id, alive, n, alive_by_id);
