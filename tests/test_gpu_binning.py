@@ -29,3 +29,18 @@ def test_shuffled_particles(n, precision):
         assert np.array_equal(c, co)
         assert neighbor_sets(c, l) == neighbor_sets(co, lo)
         d.move_boundary_rigid(0, s.boundary.shape[0], None, (0.0, 0.0, 0.0), (0.0, 0.0, 0.0), None)
+
+
+@pytest.mark.parametrize("n", [1, 513, 4097])
+def test_search_applies_uploaded_velocities(n):
+    """Velocities uploaded with the positions are in place after a search that re-orders the particles."""
+    r, rng = 0.025, np.random.default_rng(n)
+    size = np.array((2.4, 0.5, 0.9))
+    x = rng.uniform(4 * r, size - 4 * r, (n, 3)).astype(np.float32)
+    walls = box_wall((0, 0, 0), tuple(size), 2 * r).astype(np.float32)
+    d = DFSPHCUDA(Scene(config=Configuration(particleRadius=r), fluid=x, boundary=walls), neighbor_capacity=96)
+    for _ in range(3):
+        x2, v2 = rng.permutation(x), rng.uniform(-1, 1, (n, 3)).astype(np.float32)
+        d.update_fluid(x2, v2)
+        d.neighbors_search()
+        assert np.array_equal(d.velocities(), v2) and np.array_equal(d.positions(), x2)
