@@ -828,7 +828,7 @@ public:
             DF_CUDA(cudaMemsetAsync(bforce_fx, 0, (size_t)nb * 3 * sizeof(unsigned long long), stream));
         if (!n) return DFSPH_OK;
         DF_TRY(bin_fluid(true));
-        launch_build_neighbors<Real>(ds, n, ftab, btab, bnear, stream, bshifted);
+        build_lists();
         launches += 1;
         DF_TRY(flush_pending());  // velocities uploaded during the binning and the build
         if (corrupt_neighbor) {  // checked builds only (the key is rejected otherwise); one search
@@ -842,6 +842,11 @@ public:
         }
         DF_CUDA(cudaGetLastError());
         return DFSPH_OK;
+    }
+
+    void build_lists() {
+        launch_build_neighbors<Real>(ds, n, ftab, btab, bnear, stream, bshifted);
+        coef_ok = false;  // the coefficients belong to the lists
     }
 
     // Cell keys -> stable radix sort -> reorder (double buffer) -> cell table of the fluid. With
@@ -2967,7 +2972,7 @@ public:
 
     void launch_kernel(int k) {
         switch (k) {
-            case DFSPH_K_NEIGHBOR_BUILD: launch_build_neighbors<Real>(ds, n, ftab, btab, bnear, stream, bshifted); break;
+            case DFSPH_K_NEIGHBOR_BUILD: build_lists(); break;
             case DFSPH_K_DENSITY_ALPHA: density_pass(false, false); break;
             case DFSPH_K_DIVERGENCE_JACOBI: launch_divergence_jacobi<Real>(ds, n, 0, false, stream); break;
             case DFSPH_K_DIVERGENCE_RESIDUAL:
