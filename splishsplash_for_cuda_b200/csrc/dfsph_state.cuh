@@ -80,8 +80,8 @@ template <class Real> __device__ __forceinline__ void publish_state(DevState<Rea
 }
 
 // Cell keys and the histograms of their first `passes` 8-bit digits (added to hist).
-// clear0 / clear1 (words0 / words1 32-bit words each, may be null / 0): buffers the same launch sets
-// to zero (the cell table and the sort's workspace before a binning).
+// clear0 / clear1 (words0 / words1 32-bit words each, 16-byte aligned): buffers the same launch sets to
+// zero (the cell table and the sort's workspace before a binning).
 template <class Real>
 void launch_cell_keys(const Vec4<Real>* pos, uint32_t n, const StepParams<Real>& p, uint32_t* keys, uint32_t* status,
                       uint32_t* hist, int passes, cudaStream_t s, uint32_t* clear0, size_t words0, uint32_t* clear1,
