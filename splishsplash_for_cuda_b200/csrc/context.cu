@@ -108,12 +108,12 @@ public:
     uint4* nbr = nullptr;
     Vec4<Real>* coef = nullptr;
     Real* vol = nullptr;
-    bool hist_zero = false;  // the sort's histograms are zero (the last fluid reorder cleared them)
+    bool hist_zero = false;  // the sort's histograms are zero (the end of the last binning cleared them)
     bool coef_ok = false;  // the pair coefficients match the lists and the current positions
     SortBuffers sb;
     uint2* ftab = nullptr;
     uint2* btab = nullptr;
-    uint8_t* bnear = nullptr;  // per cell: a boundary particle within two cells
+    uint8_t* bnear = nullptr;  // per cell: a boundary particle within two cells; behind btab, in its allocation
     size_t cells = 0;
     Vec4<Real>* bpos[2] = {nullptr, nullptr};
     Vec4<Real>* bvel[2] = {nullptr, nullptr};
@@ -341,7 +341,7 @@ public:
         }
         f(density); f(factor); f(densityAdv); f(kcoef); f(acc); f(counts); f(nbr); f(coef); f(vol); f(bid); f(bforce); f(bforce_fx);
         f(sb.keys_a); f(sb.keys_b); f(sb.vals_a); f(sb.vals_b); f(sb.workspace);
-        f(partials); f(cfl_partials); f(readback); f(stage); f(dl); f(ds); f(ftab); f(btab); f(bnear);
+        f(partials); f(cfl_partials); f(readback); f(stage); f(dl); f(ds); f(ftab); f(btab);
         for (int b = 0; b < 2; ++b) {
             f(kappaT[b]); f(kappaVT[b]);
         }
@@ -528,16 +528,13 @@ public:
         if (c != cells) {
             if (ftab) cudaFree(ftab);
             if (btab) cudaFree(btab);
-            if (bnear) cudaFree(bnear);
             ftab = btab = nullptr;
-            bnear = nullptr;
             DF_TRY(dalloc(&ftab, c));
-            DF_TRY(dalloc(&btab, c));
-            DF_TRY(dalloc(&bnear, c));
+            DF_TRY(dalloc(&btab, c + (c + 7) / 8));  // and the byte per cell of bnear
+            bnear = reinterpret_cast<uint8_t*>(btab + c);
             cells = c;
         }
-        DF_CUDA(cudaMemsetAsync(btab, 0, cells * sizeof(uint2), stream));
-        DF_CUDA(cudaMemsetAsync(bnear, 0, cells, stream));
+        DF_CUDA(cudaMemsetAsync(btab, 0, boundary_table_words() * sizeof(uint32_t), stream));
         grid_ready = true;
         return DFSPH_OK;
     }
@@ -567,8 +564,10 @@ public:
         return true;
     }
 
-    // Zeroes the sort's histograms before a key pass, unless the last fluid reorder has (a boundary sort, or
-    // a binning that returned early, leaves its counts there).
+    // 32-bit words of btab and bnear.
+    size_t boundary_table_words() const { return 2 * (cells + (cells + 7) / 8); }
+    // Zeroes the sort's histograms before a key pass, unless the last binning has (one that returned early
+    // leaves its counts there).
     int zero_histograms() {
         if (!hist_zero) DF_CUDA(cudaMemsetAsync(sort_histograms(sb), 0, kSortHistWords * sizeof(uint32_t), stream));
         hist_zero = false;
@@ -579,14 +578,14 @@ public:
         const StepParams<Real> p = params();
         DF_TRY(zero_histograms());
         launch_cell_keys<Real>(bpos[1], nb, p, sb.keys_a, status + 1, sort_histograms(sb), key_passes, stream,
-                               (uint32_t*)btab, 2 * cells, sort_clear_begin(sb), sort_clear_words(nb, key_passes));
+                               (uint32_t*)btab, boundary_table_words(), sort_clear_begin(sb),
+                               sort_clear_words(nb, key_passes));
         uint32_t *skeys, *perm;
         radix_sort_pairs(sb, nb, key_passes, true, stream, status, &launches, &skeys, &perm);
         launch_reorder_boundary<Real>(perm, nb, bpos[1], bvel[1], bpos[0], bvel[0], bid, stream);
-        launch_cell_bounds(skeys, nb, dim[0], dim[1], dim[2], btab, stream);
-        DF_CUDA(cudaMemsetAsync(bnear, 0, cells, stream));
-        launch_mark_near_boundary(skeys, nb, dim[0], dim[1], dim[2], bnear, stream);
-        launches += 4;
+        launch_boundary_cells(skeys, nb, dim[0], dim[1], dim[2], btab, bnear, sort_histograms(sb), stream);
+        hist_zero = nb > 0;
+        launches += 3;
         if (compute_psi) {
             launch_boundary_psi<Real>(bpos[0], bpos[1], nb, p, btab, status, stream);
             DF_CUDA(cudaMemcpyAsync(bpos[0], bpos[1], (size_t)nb * sizeof(Vec4<Real>), cudaMemcpyDeviceToDevice,

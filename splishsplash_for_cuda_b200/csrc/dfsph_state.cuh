@@ -96,11 +96,10 @@ void launch_reorder_fluid(const uint32_t* perm, const uint32_t* sorted_keys, uin
 template <class Real>
 void launch_reorder_pair(const uint32_t* perm, uint32_t n, const Real* a_in, const Real* b_in, Real* a_out,
                          Real* b_out, cudaStream_t s);
-void launch_cell_bounds(const uint32_t* sorted_keys, uint32_t n, int dim_x, int dim_y, int dim_z, uint2* table,
-                        cudaStream_t s);
-// near_boundary[cell] = 1 for the cells within two cells of a boundary particle's (cleared by the caller).
-void launch_mark_near_boundary(const uint32_t* sorted_keys, uint32_t nb, int dim_x, int dim_y, int dim_z,
-                               uint8_t* near_boundary, cudaStream_t s);
+// The cell table of the sorted boundary, near_boundary[cell] = 1 for the cells within two cells of a boundary
+// particle's (both cleared by the caller), and the sort's histograms cleared (kSortHistWords words).
+void launch_boundary_cells(const uint32_t* sorted_keys, uint32_t nb, int dim_x, int dim_y, int dim_z, uint2* table,
+                           uint8_t* near_boundary, uint32_t* hist, cudaStream_t s);
 template <class Real>
 void launch_build_neighbors(const DevState<Real>* d, uint32_t n, const uint2* fluid_table, const uint2* boundary_table,
                             const uint8_t* near_boundary, cudaStream_t s, bool boundary_shifted = false);

@@ -41,8 +41,9 @@ __device__ __forceinline__ uint32_t cell_linear(int cx, int cy, int cz, int dim_
 // blocks add to the global histograms.
 // The pass clears two buffers of the binning on the way (16-byte aligned). Few particles in a large domain
 // have a table far larger than their keys: blocks are added until a thread clears no more than kClearPerThread
-// words, up to kClearBlocks blocks (the resident ones). 1000 particles, keys alone -> so: binning with 200^3 cells 792 -> 34 us,
-// 400^3 5690 -> 118 us, 20^3 unchanged; with 512 keys for every 4096 words or more it is the keys' grid.
+// words, up to kClearBlocks blocks (the resident ones). 1000 particles, a grid by the keys alone -> this one:
+// binning with 200^3 cells 792 -> 34 us, with 400^3 5690 -> 118 us, with 20^3 unchanged. Where there are 512
+// keys or more to 4096 words the two grids are the same.
 constexpr uint32_t kKeysPerThread = 2;
 constexpr size_t kClearPerThread = 16;
 constexpr size_t kClearBlocks = 148 * 8;
@@ -97,12 +98,6 @@ __device__ __forceinline__ void mark_cell_bounds(const uint32_t* __restrict__ ke
     const uint32_t lin = cell_linear((int)cx, (int)cy, (int)cz, dim_x, dim_y);
     if (i == 0 || keys[i - 1] != k) table[lin].x = i;
     if (i == n - 1 || keys[i + 1] != k) table[lin].y = i + 1;
-}
-__global__ void __launch_bounds__(kBlock) cell_bounds_kernel(const uint32_t* __restrict__ keys, uint32_t n, int dim_x,
-                                                             int dim_y, int dim_z, uint2* __restrict__ table) {
-    DFSPH_PDL_ENTER;
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) mark_cell_bounds(keys, n, i, dim_x, dim_y, dim_z, table);
 }
 
 // The end of a fluid binning in one launch: the reorder of the particles, the cell table, the state block
@@ -373,15 +368,22 @@ __global__ void __launch_bounds__(kBlock, kBuildMinBlocks) build_neighbors_kerne
     ds->counts[i] = nf | (nb << 16);
 }
 
-// Marks the cells within two cells (along each axis) of a cell that holds boundary particles: fluid in
-// an unmarked cell has no boundary neighbours, and the neighbour build skips their cell table. One
-// thread per boundary particle; the first of each cell's run marks.
-__global__ void __launch_bounds__(kBlock) mark_near_boundary_kernel(const uint32_t* __restrict__ keys, uint32_t nb,
-                                                                    int dim_x, int dim_y, int dim_z,
-                                                                    uint8_t* __restrict__ bnear) {
+// The end of a boundary binning in one launch: the cell table, the marks of the cells within two cells
+// (along each axis) of a cell that holds boundary particles, and the sort's histograms cleared for the next key
+// pass. Fluid in an unmarked cell has no boundary neighbours, and the neighbour build skips their cell table.
+// One thread per boundary particle; the first of each cell's run marks. Two launches and two memsets -> one
+// launch: moving a part of the boundary 59 -> 46 us at 500 samples, 62 -> 53 us at 23 k, 74 -> 65 us at 56 k.
+__global__ void __launch_bounds__(kBlock) boundary_cells_kernel(const uint32_t* __restrict__ keys, uint32_t nb,
+                                                                int dim_x, int dim_y, int dim_z,
+                                                                uint2* __restrict__ table,
+                                                                uint8_t* __restrict__ bnear,
+                                                                uint32_t* __restrict__ hist) {
     DFSPH_PDL_ENTER;
     const uint32_t b = blockIdx.x * blockDim.x + threadIdx.x;
+    if (blockIdx.x == gridDim.x - 1)
+        for (uint32_t k = threadIdx.x; k < kSortHistWords; k += kBlock) hist[k] = 0u;
     if (b >= nb) return;
+    mark_cell_bounds(keys, nb, b, dim_x, dim_y, dim_z, table);
     const uint32_t k = keys[b];
     if (k == kEscapedKey || (b > 0 && keys[b - 1] == k)) return;
     const int cx = (int)compact_bits10(k), cy = (int)compact_bits10(k >> 1), cz = (int)compact_bits10(k >> 2);
@@ -488,13 +490,11 @@ void launch_reorder_pair(const uint32_t* perm, uint32_t n, const Real* a_in, con
                          Real* b_out, cudaStream_t s) {
     if (n) launch_pdl(reorder_pair_kernel<Real>, grid_for(n), kBlock, 0, s, perm, n, a_in, b_in, a_out, b_out);
 }
-void launch_cell_bounds(const uint32_t* sorted_keys, uint32_t n, int dim_x, int dim_y, int dim_z, uint2* table,
-                        cudaStream_t s) {
-    if (n) launch_pdl(cell_bounds_kernel, grid_for(n), kBlock, 0, s, sorted_keys, n, dim_x, dim_y, dim_z, table);
-}
-void launch_mark_near_boundary(const uint32_t* sorted_keys, uint32_t nb, int dim_x, int dim_y, int dim_z,
-                               uint8_t* near_boundary, cudaStream_t s) {
-    if (nb) launch_pdl(mark_near_boundary_kernel, grid_for(nb), kBlock, 0, s, sorted_keys, nb, dim_x, dim_y, dim_z, near_boundary);
+void launch_boundary_cells(const uint32_t* sorted_keys, uint32_t nb, int dim_x, int dim_y, int dim_z, uint2* table,
+                           uint8_t* near_boundary, uint32_t* hist, cudaStream_t s) {
+    if (nb)
+        launch_pdl(boundary_cells_kernel, grid_for(nb), kBlock, 0, s, sorted_keys, nb, dim_x, dim_y, dim_z, table,
+                   near_boundary, hist);
 }
 template <class Real>
 void launch_build_neighbors(const DevState<Real>* d, uint32_t n, const uint2* fluid_table, const uint2* boundary_table,

@@ -73,3 +73,26 @@ def test_few_particles_in_a_large_domain():
         small.move_boundary(b)
     small.close()
     large.close()
+
+
+@pytest.mark.parametrize("precision", [32, 64])
+@pytest.mark.parametrize("n", [1, 513, 4097])
+def test_fluid_and_boundary_binnings_alternate(n, precision):
+    """Both sets are sorted with the same buffers: searches between re-binnings of the boundary at its
+    unchanged positions (a part of it moved by nothing, and all of it uploaded again) find the same sets."""
+    r, rng = 0.025, np.random.default_rng(n)
+    size = np.array((2.4, 0.5, 0.9))
+    x = rng.uniform(4 * r, size - 4 * r, (n, 3)).astype(np.float32)
+    walls = rng.permutation(box_wall((0, 0, 0), tuple(size), 2 * r).astype(np.float32))
+    s = Scene(config=Configuration(particleRadius=r), fluid=x, boundary=walls)
+    d = DFSPHCUDA(s, precision=precision, neighbor_capacity=96)
+    co, lo = Oracle(s, 64).neighbors(row=96)
+    part = lambda: d.move_boundary_rigid(0, walls.shape[0] - 1, None, (0.0, 0.0, 0.0), (0.0, 0.0, 0.0), None)
+    for bins in ((), (part,), (lambda: d.move_boundary(walls),), (part, part, lambda: d.move_boundary(walls)), ()):
+        for again in bins:
+            again()
+        d.neighbors_search()
+        c, l = d.neighbors(96)
+        assert d.status() & (_capi.ST_NEIGHBOR_OVERFLOW | _capi.ST_SORT_TIMEOUT | _capi.ST_ESCAPED) == 0
+        assert np.array_equal(c, co)
+        assert neighbor_sets(c, l) == neighbor_sets(co, lo)
