@@ -1714,7 +1714,7 @@ public:
     // Both of these for a pass that no density pass at these positions precedes.
     void ensure_coefficients() {
         if (coef_ok || !n) return;
-        launch_density_alpha<Real>(ds, n, false, false, stream, true);
+        launch_pair_coefficients<Real>(ds, n, stream);
         launches += 1;
         coef_ok = true;
     }
@@ -1786,7 +1786,10 @@ public:
 
     int external_forces(bool cfl) {
         if (!n) return DFSPH_OK;
-        ensure_coefficients();
+        if (!coef_ok) {  // the viscosity pass reads m / rho only
+            launch_volumes<Real>(ds, n, stream);
+            launches += 1;
+        }
         launch_viscosity<Real>(ds, n, cfl, stream);
         launches += 1;
         vel_updated = false;

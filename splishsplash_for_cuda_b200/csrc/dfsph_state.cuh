@@ -122,12 +122,13 @@ void launch_scatter_by_id(const uint32_t* id, uint32_t n, const Real* src, int c
                           cudaStream_t s);
 
 // ---- launch wrappers (solver.cu) ------------------------------------------------------------------
-// warm_v: scale kappa_v into the reference warm start; features: write the MLP inputs instead;
-// rows_only: write the pair coefficients and m / rho alone (for a pass that no density pass at these
-// positions precedes).
+// warm_v: scale kappa_v into the reference warm start; features: write the MLP inputs instead.
 template <class Real>
-void launch_density_alpha(const DevState<Real>* d, uint32_t n, bool warm_v, bool features, cudaStream_t s,
-                          bool rows_only = false);
+void launch_density_alpha(const DevState<Real>* d, uint32_t n, bool warm_v, bool features, cudaStream_t s);
+// What the density pass leaves for the other passes, where none at these positions precedes them: the pair
+// coefficients and m / rho, or m / rho alone.
+template <class Real> void launch_pair_coefficients(const DevState<Real>* d, uint32_t n, cudaStream_t s);
+template <class Real> void launch_volumes(const DevState<Real>* d, uint32_t n, cudaStream_t s);
 // kw: warm-start coefficients (null = kappa_v); vout: output velocities (null = in place).
 template <class Real>
 void launch_divergence_warm_jacobi(const DevState<Real>* d, uint32_t n, const Real* kw, Vec4<Real>* vout,

@@ -408,12 +408,11 @@ __device__ __forceinline__ void visit_coefficients(const uint4* __restrict__ idx
 
 // ---------------------------------------------------------------------------------------------
 // density + alpha + divergence source (+ kappa_v warm-start scaling), one pass over the neighbours.
-// warm_v, features and rows_only are runtime flags so that every mode runs the same machine code for
-// the density, alpha and pair arithmetic (the learned mode with a plain warm start reproduces the plain
-// mode bit for bit, and rebuilt coefficients are those of the density pass).
+// warm_v and features are runtime flags so that every mode runs the same machine code for the density
+// and alpha arithmetic (the learned mode with a plain warm start reproduces the plain mode bit for bit).
 template <class Real>
 __global__ void __launch_bounds__(kBlock, kGatherMinBlocks) density_alpha_kernel(const DevState<Real>* __restrict__ ds, uint32_t n,
-                                                                               bool warm_v, bool features, bool rows_only) {
+                                                                               bool warm_v, bool features) {
     DFSPH_PDL_ENTER;
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
@@ -484,10 +483,6 @@ __global__ void __launch_bounds__(kBlock, kGatherMinBlocks) density_alpha_kernel
                 return f;
             });
     }
-    if (rows_only) {
-        ds->vol[i] = xi.w / (p.density0 + ds->density[i]);
-        return;
-    }
     const Real gx = gpi.x.value(), gy = gpi.y.value(), gz = gpi.z.value();
     const Real sg = sgk.value() + (gx * gx + gy * gy + gz * gz);
     const Real alpha = -p.inv_h / rmax<Real>(sg, Real(kEps));
@@ -505,6 +500,40 @@ __global__ void __launch_bounds__(kBlock, kGatherMinBlocks) density_alpha_kernel
                            (float)ds->kappaT[i]);
         f[1] = make_float4((float)ds->kappaVT[i], 0.0f, 0.0f, 0.0f);
     }
+}
+
+// The pair coefficients alone, for a solve that no density pass at these positions precedes: the same bits
+// (every rounding of pair_factor is explicit), without the density's FP64 terms and the velocities' gathers.
+// The density pass run for its coefficients -> this: a pressure solve of two iterations 271 -> 238 us at 250 k
+// particles, 833 -> 705 us at 1 M, 737 -> 610 us at 250 k in FP64; external forces alone (volumes_kernel)
+// 104 -> 48, 329 -> 131 and 291 -> 117 us.
+template <class Real>
+__global__ void __launch_bounds__(kBlock, kGatherMinBlocks) pair_coefficients_kernel(const DevState<Real>* __restrict__ ds, uint32_t n) {
+    DFSPH_PDL_ENTER;
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const StepParams<Real>& p = ds->p;
+    const uint32_t stride = p.nbr_stride;
+    const Cubic<Real> K = p.kern;
+    const Vec4<Real> xi = ds->pos[i];
+    const uint32_t c = ds->counts[i];
+    const uint32_t nf = fluid_count(c), nb = boundary_count(c);
+    Vec4<Real> xj[2];
+    auto rows = [&](const Vec4<Real>* __restrict__ src, size_t at, uint32_t entries) {
+        visit_coefficients<Real>(
+            ds->nbr + at, ds->coef + at, stride, entries, [&](int u, uint32_t j) { xj[u] = ld4<Real>(src + j); },
+            [&](int u) { return K.pair_factor(xi.x - xj[u].x, xi.y - xj[u].y, xi.z - xj[u].z); });
+    };
+    rows(ds->pos, i, nf);
+    if (nb) rows(ds->bpos, (size_t)slot_groups(nf) * stride + i, nb);
+    ds->vol[i] = xi.w / (p.density0 + ds->density[i]);
+}
+// m / rho alone, for a viscosity pass that no density pass precedes.
+template <class Real>
+__global__ void __launch_bounds__(kBlock) volumes_kernel(const DevState<Real>* __restrict__ ds, uint32_t n) {
+    DFSPH_PDL_ENTER;
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) ds->vol[i] = ds->pos[i].w / (ds->p.density0 + ds->density[i]);
 }
 
 // Divergence warm start (divergenceSolveParticle<true>, only where the source is positive,
@@ -1126,10 +1155,15 @@ __global__ void __launch_bounds__(kBlock) gather_training_kernel(const DevState<
 }  // namespace
 
 template <class Real>
-void launch_density_alpha(const DevState<Real>* d, uint32_t n, bool warm_v, bool features, cudaStream_t s,
-                          bool rows_only) {
+void launch_density_alpha(const DevState<Real>* d, uint32_t n, bool warm_v, bool features, cudaStream_t s) {
     if (!n) return;
-    launch_pdl(density_alpha_kernel<Real>, grid_for(n), kBlock, 0, s, d, n, warm_v && !features, features, rows_only);
+    launch_pdl(density_alpha_kernel<Real>, grid_for(n), kBlock, 0, s, d, n, warm_v && !features, features);
+}
+template <class Real> void launch_pair_coefficients(const DevState<Real>* d, uint32_t n, cudaStream_t s) {
+    if (n) launch_pdl(pair_coefficients_kernel<Real>, grid_for(n), kBlock, 0, s, d, n);
+}
+template <class Real> void launch_volumes(const DevState<Real>* d, uint32_t n, cudaStream_t s) {
+    if (n) launch_pdl(volumes_kernel<Real>, grid_for(n), kBlock, 0, s, d, n);
 }
 template <class Real>
 void launch_divergence_warm_jacobi(const DevState<Real>* d, uint32_t n, const Real* kw, Vec4<Real>* vout,
@@ -1238,7 +1272,9 @@ template <class Real> void launch_cfl(DevState<Real>* d, uint32_t n_blocks, cons
 }
 
 #define DFSPH_INSTANTIATE_SOLVER(R)                                                                                  \
-    template void launch_density_alpha<R>(const DevState<R>*, uint32_t, bool, bool, cudaStream_t, bool);            \
+    template void launch_density_alpha<R>(const DevState<R>*, uint32_t, bool, bool, cudaStream_t);                  \
+    template void launch_pair_coefficients<R>(const DevState<R>*, uint32_t, cudaStream_t);                           \
+    template void launch_volumes<R>(const DevState<R>*, uint32_t, cudaStream_t);                                     \
     template void launch_divergence_warm_jacobi<R>(const DevState<R>*, uint32_t, const R*, Vec4<R>*, cudaStream_t,  \
                                                    bool);                                                            \
     template void launch_warm_values<R>(const DevState<R>*, uint32_t, int, bool, bool, double, cudaStream_t);       \

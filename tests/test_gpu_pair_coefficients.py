@@ -86,3 +86,27 @@ def test_coefficients_follow_rebuilt_lists(precision, seed):
         # bytes: alpha is scaled a second time here, and the solve may run off to NaN
         out.append((its, d.field("velocity", np.float64).tobytes(), d.field("kappa", np.float64).tobytes()))
     assert out[0] == out[1]
+
+
+@pytest.mark.parametrize("precision", [32, 64])
+@pytest.mark.parametrize("n", [1, 2, 31, 33, 130, 257, 1025])
+def test_passes_without_a_density_pass(n, precision):
+    """external_forces and pressure_solve after a change that voids what the density pass left for them:
+    the same bits as with it, over the list remainders."""
+    out = []
+    for touch in (False, True):
+        s = _sparse_block(n, seed=n)
+        d = DFSPHCUDA(s, precision=precision)
+        void = (lambda: d.set_param("viscosity", d.get_param("viscosity"))) if touch else (lambda: None)
+        d.neighbors_search()
+        d.divergence_solve()
+        void()
+        d.external_forces()
+        d.update_time_step(0.001)
+        void()
+        d.update_vel()
+        its = d.pressure_solve()
+        d.external_forces()  # with what the pressure solve has formed
+        out.append((its, d.field("velocity", np.float64).tobytes(), d.field("kappa", np.float64).tobytes(),
+                    d.field("acceleration", np.float64).tobytes()))
+    assert out[0] == out[1]
