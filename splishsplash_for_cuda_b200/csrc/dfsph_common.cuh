@@ -248,12 +248,18 @@ template <class Real> struct Cubic {
     // The same with every rounding explicit: the compiler contracts grad_factor's multiplications and
     // additions into FMAs differently from kernel to kernel. The solver passes use this one (as pair
     // coefficients), whose bits are those the passes got when each evaluated the kernel itself; the
-    // density pass keeps grad_factor for its own sums for the same reason, because the sign of its
+    // FP32 density pass keeps grad_factor for its own sums for the same reason, because the sign of its
     // divergence source switches the warm start of a particle on or off.
     __device__ __forceinline__ Real pair_factor(Real rx, Real ry, Real rz) const {
+        Real w;
+        return pair_factor(rx, ry, rz, w);
+    }
+    // And w = W(r) from the same q.
+    __device__ __forceinline__ Real pair_factor(Real rx, Real ry, Real rz, Real& w) const {
         const Real r2 = dot3(rx, ry, rz, rx, ry, rz);
         const Real inv_rl = rsqrt_(r2);
         const Real q = mul_rn(mul_rn(r2, inv_rl), invH);
+        w = r2 > Real(1e-12) ? W_of_q(q) : W0;
         const Real g = Real(1) - q;
         const Real c = (q <= Real(0.5)) ? mul_rn(mul_rn(l, q), fma(Real(3), q, Real(-2))) : mul_rn(l, mul_rn(-g, g));
         const Real f = mul_rn(mul_rn(c, inv_rl), invH);

@@ -410,9 +410,14 @@ __device__ __forceinline__ void visit_coefficients(const uint4* __restrict__ idx
 // density + alpha + divergence source (+ kappa_v warm-start scaling), one pass over the neighbours.
 // warm_v and features are runtime flags so that every mode runs the same machine code for the density
 // and alpha arithmetic (the learned mode with a plain warm start reproduces the plain mode bit for bit).
+// The FP64 build evaluates the kernel once a pair and runs two blocks an SM: at four (64 registers a thread) it
+// spills 480 bytes, at three 224, at two (124 registers) nothing. Three evaluations and four blocks -> one
+// and four -> three -> two: 180 -> 174 -> 152 -> 100 us at 250 k particles, 588 -> 545 -> 475 -> 328 us at
+// 1 M, 57 -> 52 -> 49 -> 28 us at 27 k. The FP32 build spills 8 bytes at four.
+template <class Real> constexpr int kDensityMinBlocks = std::is_same<Real, double>::value ? 2 : kGatherMinBlocks;
 template <class Real>
-__global__ void __launch_bounds__(kBlock, kGatherMinBlocks) density_alpha_kernel(const DevState<Real>* __restrict__ ds, uint32_t n,
-                                                                               bool warm_v, bool features) {
+__global__ void __launch_bounds__(kBlock, kDensityMinBlocks<Real>) density_alpha_kernel(
+    const DevState<Real>* __restrict__ ds, uint32_t n, bool warm_v, bool features) {
     DFSPH_PDL_ENTER;
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
@@ -447,8 +452,8 @@ __global__ void __launch_bounds__(kBlock, kGatherMinBlocks) density_alpha_kernel
         }
     };
     add_term(Real(0), Real(0), Real(0), xi.w, K.W0);
-    auto accumulate = [&](const Vec4<Real>& xj, Real vx, Real vy, Real vz, Real rx, Real ry, Real rz, Real f) {
-        add_term(rx, ry, rz, xj.w, kF64Terms ? Real(0) : K.W(rx, ry, rz));
+    auto accumulate = [&](const Vec4<Real>& xj, Real vx, Real vy, Real vz, Real rx, Real ry, Real rz, Real w, Real f) {
+        add_term(rx, ry, rz, xj.w, w);
         const Real gx = f * rx, gy = f * ry, gz = f * rz;
         const Real px = xj.w * gx, py = xj.w * gy, pz = xj.w * gz;
         sgk.add(px * px + py * py + pz * pz);
@@ -465,8 +470,15 @@ __global__ void __launch_bounds__(kBlock, kGatherMinBlocks) density_alpha_kernel
             },
             [&](int u) {
                 const Real rx = xi.x - xj[u].x, ry = xi.y - xj[u].y, rz = xi.z - xj[u].z;
-                accumulate(xj[u], vj[u].x, vj[u].y, vj[u].z, rx, ry, rz, K.grad_factor(rx, ry, rz));
-                return K.pair_factor(rx, ry, rz);
+                if constexpr (kF64Terms) {
+                    accumulate(xj[u], vj[u].x, vj[u].y, vj[u].z, rx, ry, rz, Real(0), K.grad_factor(rx, ry, rz));
+                    return K.pair_factor(rx, ry, rz);
+                } else {  // W, the gradient and the coefficient from one evaluation
+                    Real w;
+                    const Real f = K.pair_factor(rx, ry, rz, w);
+                    accumulate(xj[u], vj[u].x, vj[u].y, vj[u].z, rx, ry, rz, w, f);
+                    return f;
+                }
             });
     }
     if (nb) {
@@ -478,8 +490,9 @@ __global__ void __launch_bounds__(kBlock, kGatherMinBlocks) density_alpha_kernel
             [&](int u, uint32_t j) { load_bnbr(b[u], ds->bpos, ds->bvel, j, moving); },
             [&](int u) {
                 const Real rx = xi.x - b[u].x.x, ry = xi.y - b[u].x.y, rz = xi.z - b[u].x.z;
-                const Real f = K.pair_factor(rx, ry, rz);
-                accumulate(b[u].x, b[u].vx, b[u].vy, b[u].vz, rx, ry, rz, f);
+                Real w = Real(0);
+                const Real f = kF64Terms ? K.pair_factor(rx, ry, rz) : K.pair_factor(rx, ry, rz, w);
+                accumulate(b[u].x, b[u].vx, b[u].vy, b[u].vz, rx, ry, rz, w, f);
                 return f;
             });
     }
