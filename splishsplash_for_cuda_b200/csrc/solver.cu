@@ -291,9 +291,10 @@ __device__ __forceinline__ void visit_boundary(const DevState<Real>* __restrict_
         });
 }
 // The reaction f grad W_ib on boundary particle j, as the reference adds it for dynamic bodies
-// (DFSPH_core_cuda.cu:467-477, :937-946).
+// (DFSPH_core_cuda.cu:467-477, :937-946). A fill-up slot has no gradient: no atomics for it.
 template <class Real>
 __device__ __forceinline__ void add_boundary_force(unsigned long long* bf, uint32_t j, Real f, Real gx, Real gy, Real gz) {
+    if (gx == Real(0) && gy == Real(0) && gz == Real(0)) return;
     unsigned long long* fb = bf + 3 * (size_t)j;
     add_force_fx(fb, (double)(f * gx));
     add_force_fx(fb + 1, (double)(f * gy));
