@@ -265,6 +265,10 @@ int dfsph_on_step_end(dfsph_ctx* ctx);                                    /* onS
  * solves since, "iterations_v_sum" the divergence iterations),
  * "remove_escaped" (1, default: a step with stats removes particles outside the domain box),
  * "escaped_removed" (read-only: particles removed that way so far),
+ * "pair_table" (1: the passes read the kernel gradients' coefficients from a table as large as the
+ * neighbour lists, twice that in FP64; 0: they evaluate them, to the same results, and the memory is
+ * given back. A context takes the table if at least half of the device's memory stays free with it, and
+ * drops it when another of its allocations fails; setting 1 fails with DFSPH_E_NOMEM if it does not fit),
  * "boundary_forces" (1: accumulate the fluid's force on every boundary particle in each Jacobi pass,
  * -m_i k_i psi_b grad W_ib summed over both solves of a step, as the reference does for dynamic
  * bodies; cleared by each neighbour search; summed with 64-bit fixed-point atomics in units of

@@ -106,10 +106,10 @@ public:
     Vec4<Real>* acc = nullptr;
     uint32_t* counts = nullptr;
     uint4* nbr = nullptr;
-    Vec4<Real>* coef = nullptr;
+    Vec4<Real>* coef = nullptr;  // null: no table of pair coefficients (take_table)
     Real* vol = nullptr;
     bool hist_zero = false;  // the sort's histograms are zero (the end of the last binning cleared them)
-    bool coef_ok = false;  // the pair coefficients match the lists and the current positions
+    bool coef_ok = false;  // the table (if there is one) and m / rho match the lists and the current positions
     SortBuffers sb;
     uint2* ftab = nullptr;
     uint2* btab = nullptr;
@@ -132,7 +132,9 @@ public:
     uint32_t* status = nullptr;  // [0] main word, [1] scratch
     float* cfl_partials = nullptr;
     float* stage = nullptr;      // upload staging: 7 floats per particle of max(Nc, Bc)
-    void* dl = nullptr;          // download staging: 3 doubles per particle of max(Nc, Bc)
+    // Download staging, 3 doubles per particle of max(Nc, Bc), in the same memory: downloads are ordered behind
+    // what still reads an upload (velocities pending from update_fluid are applied before any of them).
+    void* dl = nullptr;
     // What a step reads back, side by side (one copy): the loop control blocks, the dt history and the
     // status words; ctl, dtd and status point into it, h_ctl, h_dt and h_status into its pinned mirror.
     struct Readback {
@@ -257,9 +259,37 @@ public:
     template <class T> int dalloc(T** p, size_t count) {
         *p = nullptr;
         if (count == 0) count = 1;
-        DF_CUDA(cudaMalloc((void**)p, count * sizeof(T)));
+        cudaError_t e = cudaMalloc((void**)p, count * sizeof(T));
+        if (e == cudaErrorMemoryAllocation && coef) {  // the solver can do without the coefficient table
+            DF_TRY(drop_table());
+            e = cudaMalloc((void**)p, count * sizeof(T));
+        }
+        DF_CUDA(e);
         return DFSPH_OK;
     }
+
+    // The table of pair coefficients (400 B a particle in FP32 at 96 neighbours, as much as the lists) is the
+    // solver's choice: without it the passes evaluate the kernel themselves, to the same bits. It is taken at
+    // creation if at least half of the device's memory stays free with it, so that contexts, and other users of
+    // the memory, for which the device was large enough without it still fit; it is given back when another
+    // allocation of the context fails, or on request. 1 M particles: 998 B a particle and 2.15 ms a step with
+    // it, 598 B and 2.37 ms without (602 B and 2.57 ms before there was one); 4 M: 7.99 and 8.85 ms.
+    int take_table() {
+        coef_ok = false;
+        DF_TRY(invalidate_graphs());
+        DF_CUDA(cudaMalloc((void**)&coef, table_bytes()));
+        return DFSPH_OK;
+    }
+    int drop_table() {
+        if (!coef) return DFSPH_OK;
+        cudaGetLastError();  // of the allocation that failed
+        DF_CUDA(cudaStreamSynchronize(stream));
+        cudaFree(coef);
+        coef = nullptr;
+        DF_TRY(invalidate_graphs());
+        return sync_state();
+    }
+    size_t table_bytes() const { return (size_t)group_capacity(cap) * stride * sizeof(Vec4<Real>); }
 
     int init(const dfsph_scene& s) {
         sc = s;
@@ -290,7 +320,6 @@ public:
         DF_TRY(dalloc(&acc, Nc));
         DF_TRY(dalloc(&counts, Nc));
         DF_TRY(dalloc(&nbr, (size_t)group_capacity(cap) * stride));
-        DF_TRY(dalloc(&coef, (size_t)group_capacity(cap) * stride));
         DF_TRY(dalloc(&vol, Nc));
         DF_TRY(dalloc(&bid, Bc));
         DF_TRY(dalloc(&brest, (size_t)Bc * 3));
@@ -303,7 +332,7 @@ public:
         DF_TRY(dalloc(&partials, 4 * ((size_t)grid_for(nmax) + 1)));  // two pairs of sums per block at most
         DF_TRY(dalloc(&cfl_partials, grid_for(nmax) + 1));
         DF_TRY(dalloc(&stage, (size_t)nmax * 7));
-        DF_CUDA(cudaMalloc(&dl, (size_t)nmax * 3 * sizeof(double)));
+        dl = stage;
         DF_CUDA(cudaMalloc((void**)&ds, sizeof(DevState<Real>)));
         DF_TRY(dalloc(&readback, 1));
         ctl = readback->ctl;
@@ -323,6 +352,9 @@ public:
         DF_CUDA(cudaEventCreateWithFlags(&ev_vel_free, cudaEventDisableTiming));
         time_step = s.time_step;
         use_graphs = s.use_graphs != 0;
+        size_t free_bytes = 0, total_bytes = 0;
+        DF_CUDA(cudaMemGetInfo(&free_bytes, &total_bytes));
+        if (free_bytes >= table_bytes() + total_bytes / 2) DF_TRY(take_table());
         DF_TRY(sync_state());
         reset_dt();
         return DFSPH_OK;
@@ -341,7 +373,7 @@ public:
         }
         f(density); f(factor); f(densityAdv); f(kcoef); f(acc); f(counts); f(nbr); f(coef); f(vol); f(bid); f(bforce); f(bforce_fx);
         f(sb.keys_a); f(sb.keys_b); f(sb.vals_a); f(sb.vals_b); f(sb.workspace);
-        f(partials); f(cfl_partials); f(readback); f(stage); f(dl); f(ds); f(ftab); f(btab);
+        f(partials); f(cfl_partials); f(readback); f(stage); f(ds); f(ftab); f(btab);
         for (int b = 0; b < 2; ++b) {
             f(kappaT[b]); f(kappaVT[b]);
         }
@@ -459,7 +491,7 @@ public:
         hs.acc = acc;
         hs.counts = counts;
         hs.nbr = nbr;
-        hs.coef = coef;
+        hs.coef = coef ? coef : pos[1 - cur];  // (the other half of the position buffers is free until the next binning)
         hs.vol = vol;
         hs.bpos = bpos[0];
         hs.bvel = bvel[0];
@@ -1613,11 +1645,11 @@ public:
         DF_CUDA(cudaGraphConditionalHandleCreate(&handle, g, u > 0 ? 0u : 1u, cudaGraphCondAssignDefault));
         auto iteration = [&]() {
             if (kind == 0) {
-                launch_divergence_jacobi<Real>(ds, n, handle, true, stream, boundary_forces);
-                launch_divergence_residual<Real>(ds, n, false, 0.0, 0, 0, handle, true, stream, g_loop_keep);
+                launch_divergence_jacobi<Real>(ds, n, coef != nullptr, handle, true, stream, boundary_forces);
+                launch_divergence_residual<Real>(ds, n, coef != nullptr, false, 0.0, 0, 0, handle, true, stream, g_loop_keep);
             } else {
-                launch_pressure_jacobi<Real>(ds, n, handle, true, stream, boundary_forces);
-                launch_pressure_residual<Real>(ds, n, false, 0.0, 0, 0, handle, true, stream, g_loop_keep);
+                launch_pressure_jacobi<Real>(ds, n, coef != nullptr, handle, true, stream, boundary_forces);
+                launch_pressure_residual<Real>(ds, n, coef != nullptr, false, 0.0, 0, 0, handle, true, stream, g_loop_keep);
             }
         };
         g_pdl_off = true;  // graph kernel edges need no programmatic launch
@@ -1692,11 +1724,11 @@ public:
         uint32_t cont = 1;
         while (cont) {
             if (kind == 0) {
-                launch_divergence_jacobi<Real>(ds, n, 0, false, stream, boundary_forces);
-                launch_divergence_residual<Real>(ds, n, false, 0.0, 0, 0, 0, false, stream, keep);
+                launch_divergence_jacobi<Real>(ds, n, coef != nullptr, 0, false, stream, boundary_forces);
+                launch_divergence_residual<Real>(ds, n, coef != nullptr, false, 0.0, 0, 0, 0, false, stream, keep);
             } else {
-                launch_pressure_jacobi<Real>(ds, n, 0, false, stream, boundary_forces);
-                launch_pressure_residual<Real>(ds, n, false, 0.0, 0, 0, 0, false, stream, keep);
+                launch_pressure_jacobi<Real>(ds, n, coef != nullptr, 0, false, stream, boundary_forces);
+                launch_pressure_residual<Real>(ds, n, coef != nullptr, false, 0.0, 0, 0, 0, false, stream, keep);
             }
             launches += 2;
             DF_CUDA(cudaMemcpyAsync(h_ctl + kind, ctl + kind, sizeof(LoopCtl), cudaMemcpyDeviceToHost, stream));
@@ -1708,13 +1740,14 @@ public:
 
     // The density pass also writes the pair coefficients and m / rho, which the other passes read.
     void density_pass(bool warm_v, bool features_out) {
-        launch_density_alpha<Real>(ds, n, warm_v, features_out, stream);
+        launch_density_alpha<Real>(ds, n, coef ? stride : 0u, warm_v, features_out, stream);
         coef_ok = true;
     }
     // Both of these for a pass that no density pass at these positions precedes.
     void ensure_coefficients() {
         if (coef_ok || !n) return;
-        launch_pair_coefficients<Real>(ds, n, stream);
+        if (coef) launch_pair_coefficients<Real>(ds, n, stream);
+        else launch_volumes<Real>(ds, n, stream);
         launches += 1;
         coef_ok = true;
     }
@@ -1725,8 +1758,8 @@ public:
         const double eta = max_error * 0.01 * sc.density0;  // divided by the device's h in the init pass
         if (!lp) {
             density_pass(true, false);
-            launch_divergence_warm_jacobi<Real>(ds, n, nullptr, nullptr, stream, boundary_forces);
-            launch_divergence_residual<Real>(ds, n, true, eta, kMinItersV, max_iter, 0, false, stream);
+            launch_divergence_warm_jacobi<Real>(ds, n, coef != nullptr, nullptr, nullptr, stream, boundary_forces);
+            launch_divergence_residual<Real>(ds, n, coef != nullptr, true, eta, kMinItersV, max_iter, 0, false, stream);
             launches += 3;
         } else {
             const bool infer = mlp_ready && !base_only && net_useful, use = mlp_ready || base_only;
@@ -1735,13 +1768,13 @@ public:
             launch_warm_values<Real>(ds, n, 0, use, infer, damping, stream);
             launches += infer ? 3 : 2;
             if (use && probe) {  // both candidates per pass, then the selection
-                launch_warm_dual<Real>(ds, n, 0, false, stream, boundary_forces);
-                launch_residual_dual<Real>(ds, n, 0, eta, kMinItersV, max_iter, stream);
+                launch_warm_dual<Real>(ds, n, coef != nullptr, 0, false, stream, boundary_forces);
+                launch_residual_dual<Real>(ds, n, coef != nullptr, 0, eta, kMinItersV, max_iter, stream);
                 launch_select_candidate<Real>(ds, n, 0, stream);
                 launches += 3;
             } else {
-                launch_divergence_warm_jacobi<Real>(ds, n, kappaVW, nullptr, stream, boundary_forces);
-                launch_divergence_residual<Real>(ds, n, true, eta, kMinItersV, max_iter, 0, false, stream, true);
+                launch_divergence_warm_jacobi<Real>(ds, n, coef != nullptr, kappaVW, nullptr, stream, boundary_forces);
+                launch_divergence_residual<Real>(ds, n, coef != nullptr, true, eta, kMinItersV, max_iter, 0, false, stream, true);
                 launches += 2;
             }
             if (use && !probe) forced_warm |= 1u;
@@ -1759,21 +1792,21 @@ public:
         ensure_coefficients();
         const double eta = max_error * 0.01 * sc.density0;
         if (!lp) {
-            launch_pressure_warm_jacobi<Real>(ds, n, fused_vel, nullptr, nullptr, stream, boundary_forces);
-            launch_pressure_residual<Real>(ds, n, true, eta, kMinItersP, max_iter, 0, false, stream);
+            launch_pressure_warm_jacobi<Real>(ds, n, coef != nullptr, fused_vel, nullptr, nullptr, stream, boundary_forces);
+            launch_pressure_residual<Real>(ds, n, coef != nullptr, true, eta, kMinItersP, max_iter, 0, false, stream);
             launches += 2;
         } else {
             const bool infer = mlp_ready && !base_only && net_useful, use = mlp_ready || base_only;
             launch_warm_values<Real>(ds, n, 1, use, infer, damping, stream);
             launches += 1;
             if (use && probe) {
-                launch_warm_dual<Real>(ds, n, 1, fused_vel, stream, boundary_forces);
-                launch_residual_dual<Real>(ds, n, 1, eta, kMinItersP, max_iter, stream);
+                launch_warm_dual<Real>(ds, n, coef != nullptr, 1, fused_vel, stream, boundary_forces);
+                launch_residual_dual<Real>(ds, n, coef != nullptr, 1, eta, kMinItersP, max_iter, stream);
                 launch_select_candidate<Real>(ds, n, 1, stream);
                 launches += 3;
             } else {
-                launch_pressure_warm_jacobi<Real>(ds, n, fused_vel, kappaW, nullptr, stream, boundary_forces);
-                launch_pressure_residual<Real>(ds, n, true, eta, kMinItersP, max_iter, 0, false, stream, true);
+                launch_pressure_warm_jacobi<Real>(ds, n, coef != nullptr, fused_vel, kappaW, nullptr, stream, boundary_forces);
+                launch_pressure_residual<Real>(ds, n, coef != nullptr, true, eta, kMinItersP, max_iter, 0, false, stream, true);
                 launches += 2;
             }
             if (use && !probe) forced_warm |= 2u;
@@ -2830,6 +2863,10 @@ public:
         }
         else if (k == "sort_withhold_tile") sort_withheld_tile = v < 0 ? kNoWithheldTile : (uint32_t)v;
         else if (k == "remove_escaped") remove_escaped = v != 0;
+        else if (k == "pair_table") {
+            if (v != 0 && !coef) DF_TRY(take_table());
+            if (v == 0) DF_TRY(drop_table());
+        }
         else if (k == "inflow_mass") {
             DF_CHECK(v > 0 && std::isfinite(v), DFSPH_E_INVALID, "inflow_mass must be positive");
             inflow_mass = (float)v;
@@ -2891,6 +2928,7 @@ public:
             return DFSPH_OK;
         }
         if (k == "viscosity") *v = sc.viscosity;
+        else if (k == "pair_table") *v = coef ? 1.0 : 0.0;
         else if (k == "density0") *v = sc.density0;
         else if (k == "max_error") *v = sc.max_error;
         else if (k == "max_error_v") *v = sc.max_error_v;
@@ -2976,18 +3014,18 @@ public:
         switch (k) {
             case DFSPH_K_NEIGHBOR_BUILD: build_lists(); break;
             case DFSPH_K_DENSITY_ALPHA: density_pass(false, false); break;
-            case DFSPH_K_DIVERGENCE_JACOBI: launch_divergence_jacobi<Real>(ds, n, 0, false, stream); break;
+            case DFSPH_K_DIVERGENCE_JACOBI: launch_divergence_jacobi<Real>(ds, n, coef != nullptr, 0, false, stream); break;
             case DFSPH_K_DIVERGENCE_RESIDUAL:
-                launch_divergence_residual<Real>(ds, n, false, 0.0, 0, 0, 0, false, stream);
+                launch_divergence_residual<Real>(ds, n, coef != nullptr, false, 0.0, 0, 0, 0, false, stream);
                 break;
             case DFSPH_K_VISCOSITY: launch_viscosity<Real>(ds, n, false, stream); break;
             case DFSPH_K_PRESSURE_WARM_JACOBI:
-                launch_pressure_warm_jacobi<Real>(ds, n, false, nullptr, nullptr, stream);
+                launch_pressure_warm_jacobi<Real>(ds, n, coef != nullptr, false, nullptr, nullptr, stream);
                 break;
             case DFSPH_K_PRESSURE_RESIDUAL:
-                launch_pressure_residual<Real>(ds, n, false, 0.0, 0, 0, 0, false, stream);
+                launch_pressure_residual<Real>(ds, n, coef != nullptr, false, 0.0, 0, 0, 0, false, stream);
                 break;
-            case DFSPH_K_PRESSURE_JACOBI: launch_pressure_jacobi<Real>(ds, n, 0, false, stream); break;
+            case DFSPH_K_PRESSURE_JACOBI: launch_pressure_jacobi<Real>(ds, n, coef != nullptr, 0, false, stream); break;
             case DFSPH_K_UPDATE_POS:
                 launch_update_pos<Real>(ds, n, stream);
                 coef_ok = false;

@@ -344,15 +344,34 @@ template <class T> __device__ __forceinline__ auto component(const T& v, int u) 
     return u == 0 ? v.x : u == 1 ? v.y : u == 2 ? v.z : v.w;
 }
 
-// Visits the slots of `groups` groups from idx / coef on, B (2 or 4) at a time: load(u, j) issues the
-// gathers of a batch, use(u, f) consumes them in slot order. Keeping a batch of independent gathers
-// in flight per thread hides the latency that a one-at-a-time loop exposes; the next group's index
+// Visits the slots of the groups that hold `entries` entries from idx / coef on, B (2 or 4) at a time:
+// load(u, j) issues the gathers of a batch, use(u, f) consumes them in slot order. Keeping a batch of independent
+// gathers in flight per thread hides the latency that a one-at-a-time loop exposes; the next group's index
 // and coefficients are loaded before this group's gathers.
-template <int B, class Real, class Load, class Use>
+// Without a coefficient table (kTable false: it does not fit the device) factor(u) forms f from the loaded
+// slot, the same bits; fill-up slots get 0 as in the table.
+template <int B, bool kTable, class Real, class Load, class Factor, class Use>
 __device__ __forceinline__ void visit_pairs(const uint4* __restrict__ idx, const Vec4<Real>* __restrict__ coef,
-                                            uint32_t stride, uint32_t groups, Load&& load, Use&& use) {
-    if (!groups) return;
+                                            uint32_t stride, uint32_t entries, Load&& load, Factor&& factor, Use&& use) {
+    if (!entries) return;
     uint4 j = ld_group(idx);
+    if constexpr (!kTable) {
+        for (uint32_t k = 0; k < entries; k += 4) {
+            idx += stride;
+            uint4 jn;
+            if (k + 4 < entries) jn = ld_group(idx);
+#pragma unroll
+            for (int b = 0; b < 4; b += 2) {
+                load(0, component(j, b));
+                load(1, component(j, b + 1));
+                use(0, k + b < entries ? factor(0) : Real(0));
+                use(1, k + b + 1 < entries ? factor(1) : Real(0));
+            }
+            j = jn;
+        }
+        return;
+    }
+    uint32_t groups = slot_groups(entries);
     Vec4<Real> f = ld_group(coef);
     while (true) {
         idx += stride;

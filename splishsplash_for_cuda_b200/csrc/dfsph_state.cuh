@@ -27,7 +27,7 @@ template <class Real> struct DevState {
     Vec4<Real>* acc;       // non-pressure acceleration
     uint32_t* counts;      // fluid count | boundary count << 16
     uint4* nbr;            // interleaved neighbour lists, nbr[g * nbr_stride + i] (dfsph_common.cuh)
-    Vec4<Real>* coef;      // pair coefficients f of the lists at the current positions, same layout
+    Vec4<Real>* coef;      // pair coefficients f of the lists at the current positions, same layout (no table: a spare array)
     Real* vol;             // m / rho, for the viscosity pass
     // boundary, cell-sorted order
     const Vec4<Real>* bpos;  // x, y, z, psi
@@ -122,16 +122,19 @@ void launch_scatter_by_id(const uint32_t* id, uint32_t n, const Real* src, int c
                           cudaStream_t s);
 
 // ---- launch wrappers (solver.cu) ------------------------------------------------------------------
+// table: the coefficient table exists (coef not null); without it the passes form the coefficients.
+// coef_stride: nbr_stride, or 0 without a table (coef then holds one group per particle, not read).
 // warm_v: scale kappa_v into the reference warm start; features: write the MLP inputs instead.
 template <class Real>
-void launch_density_alpha(const DevState<Real>* d, uint32_t n, bool warm_v, bool features, cudaStream_t s);
+void launch_density_alpha(const DevState<Real>* d, uint32_t n, uint32_t coef_stride, bool warm_v, bool features,
+                          cudaStream_t s);
 // What the density pass leaves for the other passes, where none at these positions precedes them: the pair
 // coefficients and m / rho, or m / rho alone.
 template <class Real> void launch_pair_coefficients(const DevState<Real>* d, uint32_t n, cudaStream_t s);
 template <class Real> void launch_volumes(const DevState<Real>* d, uint32_t n, cudaStream_t s);
 // kw: warm-start coefficients (null = kappa_v); vout: output velocities (null = in place).
 template <class Real>
-void launch_divergence_warm_jacobi(const DevState<Real>* d, uint32_t n, const Real* kw, Vec4<Real>* vout,
+void launch_divergence_warm_jacobi(const DevState<Real>* d, uint32_t n, bool table, const Real* kw, Vec4<Real>* vout,
                                    cudaStream_t s, bool forces = false);
 // Warm-start candidates: which = 0 divergence (kappa_v), 1 pressure (kappa). Writes the plain
 // (reference) candidate to kappaVP / kappaP and, when learned, the learned one to kappa_v + kappaVW /
@@ -150,21 +153,21 @@ void launch_gather_training(const DevState<Real>* d, uint32_t n, uint32_t batch,
                             float* t, cudaStream_t s);
 // keep: also store the unclamped residual in residV (learned warm start).
 template <class Real>
-void launch_divergence_residual(const DevState<Real>* d, uint32_t n, bool init, double eta, int min_it, int max_it,
+void launch_divergence_residual(const DevState<Real>* d, uint32_t n, bool table, bool init, double eta, int min_it, int max_it,
                                 cudaGraphConditionalHandle h, bool use_handle, cudaStream_t s, bool keep = false);
 template <class Real>
-void launch_divergence_jacobi(const DevState<Real>* d, uint32_t n, cudaGraphConditionalHandle h, bool use_handle,
+void launch_divergence_jacobi(const DevState<Real>* d, uint32_t n, bool table, cudaGraphConditionalHandle h, bool use_handle,
                               cudaStream_t s, bool forces = false);
 template <class Real> void launch_viscosity(const DevState<Real>* d, uint32_t n, bool cfl, cudaStream_t s);
 template <class Real> void launch_update_vel(const DevState<Real>* d, uint32_t n, cudaStream_t s);
 // kw null: kappa scaled by (h/h_f)^2 and clamped (reference warm start); otherwise the given final
 // warm-start coefficients. vout: output velocities (null = in place).
 template <class Real>
-void launch_pressure_warm_jacobi(const DevState<Real>* d, uint32_t n, bool fused_vel, const Real* kw,
+void launch_pressure_warm_jacobi(const DevState<Real>* d, uint32_t n, bool table, bool fused_vel, const Real* kw,
                                  Vec4<Real>* vout, cudaStream_t s, bool forces = false);
 // keep: also store the unclamped residual in resid (learned warm start).
 template <class Real>
-void launch_pressure_residual(const DevState<Real>* d, uint32_t n, bool init, double eta, int min_it, int max_it,
+void launch_pressure_residual(const DevState<Real>* d, uint32_t n, bool table, bool init, double eta, int min_it, int max_it,
                               cudaGraphConditionalHandle h, bool use_handle, cudaStream_t s, bool keep = false);
 // Both warm-start candidates in one pass (which = 0 divergence, 1 pressure): the plain candidate
 // (kappaVP / kappaP) into velP, the learned one (kappaVW / kappaW) into vel; then their init residuals
@@ -172,13 +175,13 @@ void launch_pressure_residual(const DevState<Real>* d, uint32_t n, bool init, do
 // ctl[3]); then the selection, which installs the plain candidate if the learned one's sum |r| is
 // larger. Replaces the probe + warm-start + init + fallback sequence with three launches.
 template <class Real>
-void launch_warm_dual(const DevState<Real>* d, uint32_t n, int which, bool fused_vel, cudaStream_t s, bool forces);
+void launch_warm_dual(const DevState<Real>* d, uint32_t n, bool table, int which, bool fused_vel, cudaStream_t s, bool forces);
 template <class Real>
-void launch_residual_dual(const DevState<Real>* d, uint32_t n, int which, double eta, int min_it, int max_it,
+void launch_residual_dual(const DevState<Real>* d, uint32_t n, bool table, int which, double eta, int min_it, int max_it,
                           cudaStream_t s);
 template <class Real> void launch_select_candidate(const DevState<Real>* d, uint32_t n, int which, cudaStream_t s);
 template <class Real>
-void launch_pressure_jacobi(const DevState<Real>* d, uint32_t n, cudaGraphConditionalHandle h, bool use_handle,
+void launch_pressure_jacobi(const DevState<Real>* d, uint32_t n, bool table, cudaGraphConditionalHandle h, bool use_handle,
                             cudaStream_t s, bool forces = false);
 // A box, and where to flag (1 inside, 0 outside) and count the particles outside it (alive null: nowhere).
 struct EscapeBox {

@@ -182,6 +182,12 @@ __device__ __forceinline__ void load_bnbr(BNbr<Real>& b, const Vec4<Real>* __res
 #endif
 constexpr int kPairBatch = DFSPH_PAIR_BATCH;
 
+template <class Real>
+__device__ __forceinline__ Real pair_factor(const StepParams<Real>& p, const Vec4<Real>& a, const Vec4<Real>& b) {
+    const Cubic<Real> K = p.kern;
+    return K.pair_factor(a.x - b.x, a.y - b.y, a.z - b.z);
+}
+
 // One term m_j (v_i - v_j).grad W_ij of a divergence, grad W_ij = f (x_i - x_j).
 template <class Real>
 __device__ __forceinline__ void add_divergence(KSum<Real>& s, Real m, Real f, Real rx, Real ry, Real rz, Real dvx, Real dvy,
@@ -190,7 +196,7 @@ __device__ __forceinline__ void add_divergence(KSum<Real>& s, Real m, Real f, Re
 }
 
 // Sum over fluid then boundary neighbours of m_j (v_i - v_j).grad W_ij, in list order.
-template <class Real>
+template <bool kTable, class Real>
 __device__ __forceinline__ Real velocity_divergence(const DevState<Real>* __restrict__ ds, const StepParams<Real>& p,
                                                     uint32_t i, const Vec4<Real>& xi, const Vec4<Real>& vi,
                                                     uint32_t nf, uint32_t nb, const Vec4<Real>* __restrict__ vel) {
@@ -201,12 +207,13 @@ __device__ __forceinline__ Real velocity_divergence(const DevState<Real>* __rest
     KSum<Real> s;
     {
         Vec4<Real> xj[kPairBatch], vj[kPairBatch];
-        visit_pairs<kPairBatch, Real>(
-            idx, coef, stride, slot_groups(nf),
+        visit_pairs<kPairBatch, kTable, Real>(
+            idx, coef, stride, nf,
             [&](int u, uint32_t j) {
                 xj[u] = ld4<Real>(pos + j);
                 vj[u] = ld4<Real>(vel + j);
             },
+            [&](int u) { return pair_factor(p, xi, xj[u]); },
             [&](int u, Real f) {
                 add_divergence(s, xj[u].w, f, xi.x - xj[u].x, xi.y - xj[u].y, xi.z - xj[u].z, vi.x - vj[u].x,
                                vi.y - vj[u].y, vi.z - vj[u].z);
@@ -216,9 +223,10 @@ __device__ __forceinline__ Real velocity_divergence(const DevState<Real>* __rest
         const bool moving = p.boundary_moving != 0;
         const size_t at = (size_t)slot_groups(nf) * stride;
         BNbr<Real> b[2];
-        visit_pairs<2, Real>(
-            idx + at, coef + at, stride, slot_groups(nb),
+        visit_pairs<2, kTable, Real>(
+            idx + at, coef + at, stride, nb,
             [&](int u, uint32_t j) { load_bnbr(b[u], ds->bpos, ds->bvel, j, moving); },
+            [&](int u) { return pair_factor(p, xi, b[u].x); },
             [&](int u, Real f) {
                 add_divergence(s, b[u].x.w, f, xi.x - b[u].x.x, xi.y - b[u].x.y, xi.z - b[u].x.z, vi.x - b[u].vx,
                                vi.y - b[u].vy, vi.z - b[u].vz);
@@ -229,7 +237,7 @@ __device__ __forceinline__ Real velocity_divergence(const DevState<Real>* __rest
 
 // velocity_divergence for two velocity fields in one pass over the neighbours (positions, indices and
 // coefficients loaded once); each sum is accumulated exactly as velocity_divergence would.
-template <class Real>
+template <bool kTable, class Real>
 __device__ __forceinline__ void velocity_divergence2(const DevState<Real>* __restrict__ ds, const StepParams<Real>& p,
                                                      uint32_t i, const Vec4<Real>& xi, const Vec4<Real>& via,
                                                      const Vec4<Real>& vib, uint32_t nf, uint32_t nb,
@@ -242,13 +250,14 @@ __device__ __forceinline__ void velocity_divergence2(const DevState<Real>* __res
     KSum<Real> sa, sb;
     {
         Vec4<Real> xj[2], va[2], vb[2];
-        visit_pairs<2, Real>(
-            idx, coef, stride, slot_groups(nf),
+        visit_pairs<2, kTable, Real>(
+            idx, coef, stride, nf,
             [&](int u, uint32_t j) {
                 xj[u] = ld4<Real>(pos + j);
                 va[u] = ld4<Real>(vela + j);
                 vb[u] = ld4<Real>(velb + j);
             },
+            [&](int u) { return pair_factor(p, xi, xj[u]); },
             [&](int u, Real f) {
                 const Real rx = xi.x - xj[u].x, ry = xi.y - xj[u].y, rz = xi.z - xj[u].z;
                 add_divergence(sa, xj[u].w, f, rx, ry, rz, via.x - va[u].x, via.y - va[u].y, via.z - va[u].z);
@@ -259,9 +268,10 @@ __device__ __forceinline__ void velocity_divergence2(const DevState<Real>* __res
         const bool moving = p.boundary_moving != 0;
         const size_t at = (size_t)slot_groups(nf) * stride;
         BNbr<Real> b[2];
-        visit_pairs<2, Real>(
-            idx + at, coef + at, stride, slot_groups(nb),
+        visit_pairs<2, kTable, Real>(
+            idx + at, coef + at, stride, nb,
             [&](int u, uint32_t j) { load_bnbr(b[u], ds->bpos, ds->bvel, j, moving); },
+            [&](int u) { return pair_factor(p, xi, b[u].x); },
             [&](int u, Real f) {
                 const Real rx = xi.x - b[u].x.x, ry = xi.y - b[u].x.y, rz = xi.z - b[u].x.z;
                 add_divergence(sa, b[u].x.w, f, rx, ry, rz, via.x - b[u].vx, via.y - b[u].vy, via.z - b[u].vz);
@@ -273,19 +283,21 @@ __device__ __forceinline__ void velocity_divergence2(const DevState<Real>* __res
 }
 
 // Boundary part of a Jacobi sum: use(j, psi_b, grad W_ib) for every boundary neighbour (b = j).
-template <class Real, class Use>
-__device__ __forceinline__ void visit_boundary(const DevState<Real>* __restrict__ ds, uint32_t stride, uint32_t i,
+template <bool kTable, class Real, class Use>
+__device__ __forceinline__ void visit_boundary(const DevState<Real>* __restrict__ ds, const StepParams<Real>& p, uint32_t i,
                                                const Vec4<Real>& xi, uint32_t nf, uint32_t nb, Use&& use) {
     const Vec4<Real>* __restrict__ bpos = ds->bpos;
     Vec4<Real> xb[2];
     uint32_t jb[2];
+    const uint32_t stride = p.nbr_stride;
     const size_t at = (size_t)slot_groups(nf) * stride + i;
-    visit_pairs<2, Real>(
-        ds->nbr + at, ds->coef + at, stride, slot_groups(nb),
+    visit_pairs<2, kTable, Real>(
+        ds->nbr + at, ds->coef + at, stride, nb,
         [&](int u, uint32_t j) {
             xb[u] = ld4<Real>(bpos + j);
             jb[u] = j;
         },
+        [&](int u) { return pair_factor(p, xi, xb[u]); },
         [&](int u, Real f) {
             use(jb[u], xb[u].w, mul_rn(f, xi.x - xb[u].x), mul_rn(f, xi.y - xb[u].y), mul_rn(f, xi.z - xb[u].z));
         });
@@ -306,7 +318,7 @@ __device__ __forceinline__ void add_boundary_force(unsigned long long* bf, uint3
 // kof(j) returns k_j (a load, possibly transformed). With boundary forces on (kForces, and at run time
 // `forces`), each boundary term also adds -m_i k_i psi_b grad W_ib to the boundary particle's force.
 // A fill-up slot (f = 0) adds a zero and leaves the sum as it is.
-template <class Real, bool kForces = false, class KOf>
+template <bool kTable, bool kForces, class Real, class KOf>
 __device__ __forceinline__ void jacobi_sum(const DevState<Real>* __restrict__ ds, const StepParams<Real>& p, uint32_t i,
                                            const Vec4<Real>& xi, Real ki, uint32_t nf, uint32_t nb, KOf&& kof,
                                            KSum3<Real>& acc, bool forces = true) {
@@ -315,12 +327,13 @@ __device__ __forceinline__ void jacobi_sum(const DevState<Real>* __restrict__ ds
     {
         Vec4<Real> xj[kPairBatch];
         Real kj[kPairBatch];
-        visit_pairs<kPairBatch, Real>(
-            ds->nbr + i, ds->coef + i, stride, slot_groups(nf),
+        visit_pairs<kPairBatch, kTable, Real>(
+            ds->nbr + i, ds->coef + i, stride, nf,
             [&](int u, uint32_t j) {
                 xj[u] = ld4<Real>(pos + j);
                 kj[u] = kof(j);
             },
+            [&](int u) { return pair_factor(p, xi, xj[u]); },
             [&](int u, Real f) {
                 const Real ks = ki + kj[u];
                 if (above_eps(ks))
@@ -330,7 +343,7 @@ __device__ __forceinline__ void jacobi_sum(const DevState<Real>* __restrict__ ds
     }
     if (nb && above_eps(ki)) {
         unsigned long long* __restrict__ bf = (kForces && forces) ? ds->bforce : nullptr;
-        visit_boundary<Real>(ds, stride, i, xi, nf, nb, [&](uint32_t j, Real psi, Real gx, Real gy, Real gz) {
+        visit_boundary<kTable>(ds, p, i, xi, nf, nb, [&](uint32_t j, Real psi, Real gx, Real gy, Real gz) {
             const Real sc = mul_rn(ki, psi);
             acc.add_product(sc, gx, gy, gz);
             if (kForces && bf) add_boundary_force(bf, j, -xi.w * sc, gx, gy, gz);
@@ -342,7 +355,7 @@ __device__ __forceinline__ void jacobi_sum(const DevState<Real>* __restrict__ ds
 // coefficients ka / kb (the plain and the learned candidate), each accumulated exactly as a
 // single-candidate pass would (the gradient is shared). Boundary forces, when on, follow candidate b
 // (the one applied in place).
-template <class Real, bool kForces = false, class KOfA, class KOfB>
+template <bool kTable, bool kForces, class Real, class KOfA, class KOfB>
 __device__ __forceinline__ void jacobi_sum2(const DevState<Real>* __restrict__ ds, const StepParams<Real>& p,
                                             uint32_t i, const Vec4<Real>& xi, Real kia, Real kib, uint32_t nf,
                                             uint32_t nb, KOfA&& kofa, KOfB&& kofb, KSum3<Real>& acca,
@@ -352,13 +365,14 @@ __device__ __forceinline__ void jacobi_sum2(const DevState<Real>* __restrict__ d
     {
         Vec4<Real> xj[2];
         Real kja[2], kjb[2];
-        visit_pairs<2, Real>(
-            ds->nbr + i, ds->coef + i, stride, slot_groups(nf),
+        visit_pairs<2, kTable, Real>(
+            ds->nbr + i, ds->coef + i, stride, nf,
             [&](int u, uint32_t j) {
                 xj[u] = ld4<Real>(pos + j);
                 kja[u] = kofa(j);
                 kjb[u] = kofb(j);
             },
+            [&](int u) { return pair_factor(p, xi, xj[u]); },
             [&](int u, Real f) {
                 const Real ksa = kia + kja[u], ksb = kib + kjb[u];
                 const Real gx = mul_rn(f, xi.x - xj[u].x), gy = mul_rn(f, xi.y - xj[u].y), gz = mul_rn(f, xi.z - xj[u].z);
@@ -369,7 +383,7 @@ __device__ __forceinline__ void jacobi_sum2(const DevState<Real>* __restrict__ d
     const bool ba = above_eps(kia), bb = above_eps(kib);
     if (nb && (ba || bb)) {
         unsigned long long* __restrict__ bf = kForces ? ds->bforce : nullptr;
-        visit_boundary<Real>(ds, stride, i, xi, nf, nb, [&](uint32_t j, Real psi, Real gx, Real gy, Real gz) {
+        visit_boundary<kTable>(ds, p, i, xi, nf, nb, [&](uint32_t j, Real psi, Real gx, Real gy, Real gz) {
             if (ba) acca.add_product(mul_rn(kia, psi), gx, gy, gz);
             if (bb) {
                 const Real sc = mul_rn(kib, psi);
@@ -384,7 +398,8 @@ __device__ __forceinline__ void jacobi_sum2(const DevState<Real>* __restrict__ d
 // writes their pair coefficients, 0 for the fill-up slots.
 template <class Real, class Load, class Use>
 __device__ __forceinline__ void visit_coefficients(const uint4* __restrict__ idx, Vec4<Real>* __restrict__ coef,
-                                                   uint32_t stride, uint32_t entries, Load&& load, Use&& use) {
+                                                   uint32_t stride, uint32_t coef_stride, uint32_t entries, Load&& load,
+                                                   Use&& use) {
     if (!entries) return;
     uint4 j = ld_group(idx);
     for (uint32_t k = 0; k < entries; k += 4) {
@@ -402,7 +417,7 @@ __device__ __forceinline__ void visit_coefficients(const uint4* __restrict__ idx
         if (k + 2 < entries) f.z = use(0);
         if (k + 3 < entries) f.w = use(1);
         *coef = f;
-        coef += stride;
+        coef += coef_stride;
         j = jn;
     }
 }
@@ -416,9 +431,11 @@ __device__ __forceinline__ void visit_coefficients(const uint4* __restrict__ idx
 // and four -> three -> two: 180 -> 174 -> 152 -> 100 us at 250 k particles, 588 -> 545 -> 475 -> 328 us at
 // 1 M, 57 -> 52 -> 49 -> 28 us at 27 k. The FP32 build spills 8 bytes at four.
 template <class Real> constexpr int kDensityMinBlocks = std::is_same<Real, double>::value ? 2 : kGatherMinBlocks;
+// Without a coefficient table coef_stride is 0, and a particle's groups go one over the other into a spare array:
+// the same machine code either way, because the compiler contracts the FP32 sums of alpha as it likes.
 template <class Real>
 __global__ void __launch_bounds__(kBlock, kDensityMinBlocks<Real>) density_alpha_kernel(
-    const DevState<Real>* __restrict__ ds, uint32_t n, bool warm_v, bool features) {
+    const DevState<Real>* __restrict__ ds, uint32_t n, bool warm_v, bool features, uint32_t coef_stride) {
     DFSPH_PDL_ENTER;
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
@@ -464,7 +481,7 @@ __global__ void __launch_bounds__(kBlock, kDensityMinBlocks<Real>) density_alpha
     {
         Vec4<Real> xj[2], vj[2];
         visit_coefficients<Real>(
-            ds->nbr + i, ds->coef + i, stride, nf,
+            ds->nbr + i, ds->coef + i, stride, coef_stride, nf,
             [&](int u, uint32_t j) {
                 xj[u] = ld4<Real>(pos + j);
                 vj[u] = ld4<Real>(vel + j);
@@ -485,9 +502,9 @@ __global__ void __launch_bounds__(kBlock, kDensityMinBlocks<Real>) density_alpha
     if (nb) {
         const bool moving = p.boundary_moving != 0;
         BNbr<Real> b[2];
-        const size_t at = (size_t)slot_groups(nf) * stride + i;
+        const size_t g = slot_groups(nf);
         visit_coefficients<Real>(
-            ds->nbr + at, ds->coef + at, stride, nb,
+            ds->nbr + g * stride + i, ds->coef + g * coef_stride + i, stride, coef_stride, nb,
             [&](int u, uint32_t j) { load_bnbr(b[u], ds->bpos, ds->bvel, j, moving); },
             [&](int u) {
                 const Real rx = xi.x - b[u].x.x, ry = xi.y - b[u].x.y, rz = xi.z - b[u].x.z;
@@ -535,7 +552,7 @@ __global__ void __launch_bounds__(kBlock, kGatherMinBlocks) pair_coefficients_ke
     Vec4<Real> xj[2];
     auto rows = [&](const Vec4<Real>* __restrict__ src, size_t at, uint32_t entries) {
         visit_coefficients<Real>(
-            ds->nbr + at, ds->coef + at, stride, entries, [&](int u, uint32_t j) { xj[u] = ld4<Real>(src + j); },
+            ds->nbr + at, ds->coef + at, stride, stride, entries, [&](int u, uint32_t j) { xj[u] = ld4<Real>(src + j); },
             [&](int u) { return K.pair_factor(xi.x - xj[u].x, xi.y - xj[u].y, xi.z - xj[u].z); });
     };
     rows(ds->pos, i, nf);
@@ -552,7 +569,7 @@ __global__ void __launch_bounds__(kBlock) volumes_kernel(const DevState<Real>* _
 
 // Divergence warm start (divergenceSolveParticle<true>, only where the source is positive,
 // DFSPH_core_cuda.cu:509-512): v_i += h * sum (kv_i + kv_j) m_j grad W_ij + h kv_i sum psi_b grad W_ib.
-template <class Real, bool kForces>
+template <class Real, bool kForces, bool kTable>
 __global__ void __launch_bounds__(kBlock, kGatherMinBlocks) divergence_warm_jacobi_kernel(const DevState<Real>* __restrict__ ds,
                                                                         uint32_t n, const Real* __restrict__ kw,
                                                                         Vec4<Real>* __restrict__ vout) {
@@ -569,7 +586,7 @@ __global__ void __launch_bounds__(kBlock, kGatherMinBlocks) divergence_warm_jaco
     const Vec4<Real> xi = ds->pos[i];
     const uint32_t c = ds->counts[i];
     KSum3<Real> acc;
-    jacobi_sum<Real, kForces>(ds, p, i, xi, ki, fluid_count(c), boundary_count(c), [&](uint32_t j) { return kv[j]; },
+    jacobi_sum<kTable, kForces>(ds, p, i, xi, ki, fluid_count(c), boundary_count(c), [&](uint32_t j) { return kv[j]; },
                               acc, vout == nullptr);  // a candidate pass (vout set) adds no boundary force
     Vec4<Real> v = ds->vel[i];
     v.x += acc.x.value() * p.h;
@@ -585,7 +602,7 @@ constexpr int kLoop = 0, kInitPass = 1;
 // sum psi_b (v_i - v_b).grad W_ib, 0), 0 with fewer than 20 neighbours. Also stores
 // k_i = rho_dot_i * alpha_i for the next Jacobi pass. The init pass additionally zeroes kappa_v
 // (DFSPH_divergence_init_kernel, :631-633).
-template <class Real, int kMode, bool kKeep>
+template <class Real, int kMode, bool kKeep, bool kTable>
 __global__ void __launch_bounds__(kBlock, kGatherMinBlocks) divergence_residual_kernel(const DevState<Real>* __restrict__ ds, uint32_t n,
                                                                      double eta, int min_it, int max_it,
                                                                      cudaGraphConditionalHandle handle,
@@ -608,7 +625,7 @@ __global__ void __launch_bounds__(kBlock, kGatherMinBlocks) divergence_residual_
         if (num >= kMinNeighborsForDivergence) {
             const Vec4<Real> xi = ds->pos[i];
             const Vec4<Real> vi = vel[i];
-            raw = velocity_divergence<Real>(ds, p, i, xi, vi, nf, nb, vel);
+            raw = velocity_divergence<kTable>(ds, p, i, xi, vi, nf, nb, vel);
         }
         const Real dadv = rmax<Real>(raw, Real(0));
         if (kKeep) ds->residV[i] = raw;  // learned warm start only
@@ -625,7 +642,7 @@ __global__ void __launch_bounds__(kBlock, kGatherMinBlocks) divergence_residual_
 
 // Divergence Jacobi iteration (divergenceSolveParticle<false>): k_i = rho_dot_i alpha_i,
 // kappa_v_i += k_i, v_i += h * [sum (k_i + k_j) m_j grad W_ij + k_i sum psi_b grad W_ib].
-template <class Real, bool kForces>
+template <class Real, bool kForces, bool kTable>
 __global__ void __launch_bounds__(kBlock, kGatherMinBlocks) divergence_jacobi_kernel(const DevState<Real>* __restrict__ ds, uint32_t n,
                                                                    cudaGraphConditionalHandle handle, bool use_handle) {
     DFSPH_PDL_ENTER;
@@ -641,7 +658,7 @@ __global__ void __launch_bounds__(kBlock, kGatherMinBlocks) divergence_jacobi_ke
     const Vec4<Real> xi = ds->pos[i];
     const uint32_t c = ds->counts[i];
     KSum3<Real> acc;
-    jacobi_sum<Real, kForces>(ds, p, i, xi, ki, fluid_count(c), boundary_count(c), [&](uint32_t j) { return kc[j]; },
+    jacobi_sum<kTable, kForces>(ds, p, i, xi, ki, fluid_count(c), boundary_count(c), [&](uint32_t j) { return kc[j]; },
                               acc);
     Vec4<Real> v = ds->vel[i];
     v.x += acc.x.value() * p.h;
@@ -748,7 +765,7 @@ __global__ void __launch_bounds__(kBlock) update_vel_kernel(const DevState<Real>
 // Pressure warm start (pressureSolveParticle<true>) fused with the velocity update: with
 // kFusedVel the particle first applies v_i += h a_i and uses kappa scaled by (h/h_future)^2 and
 // clamped at -0.5 (update_vel, :3061-3065), computed for the neighbours on the fly.
-template <class Real, bool kFusedVel, bool kForces>
+template <class Real, bool kFusedVel, bool kForces, bool kTable>
 __global__ void __launch_bounds__(kBlock, kGatherMinBlocks) pressure_warm_jacobi_kernel(const DevState<Real>* __restrict__ ds,
                                                                       uint32_t n, const Real* __restrict__ kw,
                                                                       Vec4<Real>* __restrict__ vout) {
@@ -765,7 +782,7 @@ __global__ void __launch_bounds__(kBlock, kGatherMinBlocks) pressure_warm_jacobi
     const Vec4<Real> xi = ds->pos[i];
     const uint32_t c = ds->counts[i];
     KSum3<Real> acc;
-    jacobi_sum<Real, kForces>(ds, p, i, xi, ki, fluid_count(c), boundary_count(c),
+    jacobi_sum<kTable, kForces>(ds, p, i, xi, ki, fluid_count(c), boundary_count(c),
                               [&](uint32_t j) { return scale ? rmax<Real>(kap[j] * r2, Real(-0.5)) : kap[j]; }, acc,
                               vout == nullptr);  // a candidate pass (vout set) adds no boundary force
     Vec4<Real> v = ds->vel[i];
@@ -784,7 +801,7 @@ __global__ void __launch_bounds__(kBlock, kGatherMinBlocks) pressure_warm_jacobi
 // Density residual (computeDensityAdv): rho_adv_i = max(rho_i + h_f * [sum m_j (v_i - v_j).grad W_ij
 // + sum psi_b (v_i - v_b).grad W_ib] - rho0, 0); kappa_i += rho_adv_i alpha_i; k_i = rho_adv_i alpha_i.
 // kInit first scales alpha by 1/h_future and zeroes kappa (DFSPH_pressure_init_kernel, :1230-1238).
-template <class Real, int kMode, bool kKeep>
+template <class Real, int kMode, bool kKeep, bool kTable>
 __global__ void __launch_bounds__(kBlock, kGatherMinBlocks) pressure_residual_kernel(const DevState<Real>* __restrict__ ds, uint32_t n,
                                                                    double eta, int min_it, int max_it,
                                                                    cudaGraphConditionalHandle handle,
@@ -806,7 +823,7 @@ __global__ void __launch_bounds__(kBlock, kGatherMinBlocks) pressure_residual_ke
         const Vec4<Real> xi = ds->pos[i];
         const Vec4<Real> vi = vel[i];
         const uint32_t c = ds->counts[i];
-        const Real sdiv = velocity_divergence<Real>(ds, p, i, xi, vi, fluid_count(c), boundary_count(c), vel);
+        const Real sdiv = velocity_divergence<kTable>(ds, p, i, xi, vi, fluid_count(c), boundary_count(c), vel);
         const Real raw = ds->density[i] + p.h_future * sdiv;  // density[] = rho - rho0
         const Real dadv = rmax<Real>(raw, Real(0));
         if (kKeep) ds->resid[i] = raw;  // learned warm start only
@@ -824,7 +841,7 @@ __global__ void __launch_bounds__(kBlock, kGatherMinBlocks) pressure_residual_ke
 
 // Pressure Jacobi iteration (pressureSolveParticle<false>): v_i += h_f * [sum (k_i + k_j) m_j grad W_ij
 // + k_i sum psi_b grad W_ib] with k = rho_adv * alpha.
-template <class Real, bool kForces>
+template <class Real, bool kForces, bool kTable>
 __global__ void __launch_bounds__(kBlock, kGatherMinBlocks) pressure_jacobi_kernel(const DevState<Real>* __restrict__ ds, uint32_t n,
                                                                  cudaGraphConditionalHandle handle, bool use_handle) {
     DFSPH_PDL_ENTER;
@@ -837,7 +854,7 @@ __global__ void __launch_bounds__(kBlock, kGatherMinBlocks) pressure_jacobi_kern
     const Vec4<Real> xi = ds->pos[i];
     const uint32_t c = ds->counts[i];
     KSum3<Real> acc;
-    jacobi_sum<Real, kForces>(ds, p, i, xi, ki, fluid_count(c), boundary_count(c), [&](uint32_t j) { return kc[j]; },
+    jacobi_sum<kTable, kForces>(ds, p, i, xi, ki, fluid_count(c), boundary_count(c), [&](uint32_t j) { return kc[j]; },
                               acc);
     Vec4<Real> v = ds->vel[i];
     v.x += acc.x.value() * p.h_future;
@@ -892,7 +909,7 @@ __global__ void __launch_bounds__(kBlock) update_pos_kernel(DevState<Real>* ds, 
 constexpr int kDualMinBlocks = DFSPH_DUAL_MIN_BLOCKS;
 // The plain candidate (kappaVP / kappaP) goes to velP, the learned one (kappaVW / kappaW) to vel in
 // place; each velocity is the one the single-candidate pass would produce.
-template <class Real, bool kForces>
+template <class Real, bool kForces, bool kTable>
 __global__ void __launch_bounds__(kBlock, kDualMinBlocks) divergence_warm_dual_kernel(
     const DevState<Real>* __restrict__ ds, uint32_t n) {
     DFSPH_PDL_ENTER;
@@ -908,7 +925,7 @@ __global__ void __launch_bounds__(kBlock, kDualMinBlocks) divergence_warm_dual_k
     const Vec4<Real> xi = ds->pos[i];
     const uint32_t c = ds->counts[i];
     KSum3<Real> acca, accb;
-    jacobi_sum2<Real, kForces>(ds, p, i, xi, ka[i], kb[i], fluid_count(c), boundary_count(c),
+    jacobi_sum2<kTable, kForces>(ds, p, i, xi, ka[i], kb[i], fluid_count(c), boundary_count(c),
                                [&](uint32_t j) { return ka[j]; }, [&](uint32_t j) { return kb[j]; }, acca, accb);
     const Vec4<Real> v0 = ds->vel[i];
     Vec4<Real> va = v0, vb = v0;
@@ -922,7 +939,7 @@ __global__ void __launch_bounds__(kBlock, kDualMinBlocks) divergence_warm_dual_k
     ds->vel[i] = vb;
 }
 
-template <class Real, bool kFusedVel, bool kForces>
+template <class Real, bool kFusedVel, bool kForces, bool kTable>
 __global__ void __launch_bounds__(kBlock, kDualMinBlocks) pressure_warm_dual_kernel(
     const DevState<Real>* __restrict__ ds, uint32_t n) {
     DFSPH_PDL_ENTER;
@@ -934,7 +951,7 @@ __global__ void __launch_bounds__(kBlock, kDualMinBlocks) pressure_warm_dual_ker
     const Vec4<Real> xi = ds->pos[i];
     const uint32_t c = ds->counts[i];
     KSum3<Real> acca, accb;
-    jacobi_sum2<Real, kForces>(ds, p, i, xi, ka[i], kb[i], fluid_count(c), boundary_count(c),
+    jacobi_sum2<kTable, kForces>(ds, p, i, xi, ka[i], kb[i], fluid_count(c), boundary_count(c),
                                [&](uint32_t j) { return ka[j]; }, [&](uint32_t j) { return kb[j]; }, acca, accb);
     Vec4<Real> v = ds->vel[i];
     if (kFusedVel) {
@@ -957,7 +974,7 @@ __global__ void __launch_bounds__(kBlock, kDualMinBlocks) pressure_warm_dual_ker
 // Init residual pass of both candidates: the learned one (vel) writes the solver's arrays and
 // reduces into ctl[slot] (sum of the clamped residuals, aux = sum |r|); the plain one (velP) writes
 // dadvP / kcP / rawP and reduces into ctl[3] the same way (separate block partials).
-template <class Real>
+template <class Real, bool kTable>
 __global__ void __launch_bounds__(kBlock, kDualMinBlocks) divergence_residual_dual_kernel(
     const DevState<Real>* __restrict__ ds, uint32_t n, double eta, int min_it, int max_it) {
     DFSPH_PDL_ENTER;
@@ -974,7 +991,7 @@ __global__ void __launch_bounds__(kBlock, kDualMinBlocks) divergence_residual_du
         Real rb = Real(0), ra = Real(0);
         if (num >= kMinNeighborsForDivergence) {
             const Vec4<Real> xi = ds->pos[i];
-            velocity_divergence2<Real>(ds, p, i, xi, ds->velP[i], ds->vel[i], nf, nb, ds->velP, ds->vel, ra, rb);
+            velocity_divergence2<kTable>(ds, p, i, xi, ds->velP[i], ds->vel[i], nf, nb, ds->velP, ds->vel, ra, rb);
         }
         const Real alpha = ds->factor[i];
         const Real db = rmax<Real>(rb, Real(0)), da = rmax<Real>(ra, Real(0));
@@ -994,7 +1011,7 @@ __global__ void __launch_bounds__(kBlock, kDualMinBlocks) divergence_residual_du
     reduce_and_decide<1, true>(ca, ds->partials + 2 * gridDim.x, ds->ctl + 3, n, eta, min_it, max_it, 0, false, aa);
 }
 
-template <class Real>
+template <class Real, bool kTable>
 __global__ void __launch_bounds__(kBlock, kDualMinBlocks) pressure_residual_dual_kernel(
     const DevState<Real>* __restrict__ ds, uint32_t n, double eta, int min_it, int max_it) {
     DFSPH_PDL_ENTER;
@@ -1008,7 +1025,7 @@ __global__ void __launch_bounds__(kBlock, kDualMinBlocks) pressure_residual_dual
         const uint32_t c = ds->counts[i];
         const uint32_t nf = fluid_count(c), nb = boundary_count(c);
         Real sa, sb;
-        velocity_divergence2<Real>(ds, p, i, xi, ds->velP[i], ds->vel[i], nf, nb, ds->velP, ds->vel, sa, sb);
+        velocity_divergence2<kTable>(ds, p, i, xi, ds->velP[i], ds->vel[i], nf, nb, ds->velP, ds->vel, sa, sb);
         const Real rb = ds->density[i] + p.h_future * sb, ra = ds->density[i] + p.h_future * sa;
         const Real db = rmax<Real>(rb, Real(0)), da = rmax<Real>(ra, Real(0));
         const Real kb = db * alpha, ka = da * alpha;
@@ -1168,10 +1185,18 @@ __global__ void __launch_bounds__(kBlock) gather_training_kernel(const DevState<
 
 }  // namespace
 
+// Calls f with the coefficient table's presence as a type: the passes are instantiated with and without it,
+// because a branch in the visit cost 1 to 5 % a pass (250 k and 1 M particles).
+template <class F> static void with_table(bool table, F&& f) {
+    if (table) f(std::true_type{});
+    else f(std::false_type{});
+}
+
 template <class Real>
-void launch_density_alpha(const DevState<Real>* d, uint32_t n, bool warm_v, bool features, cudaStream_t s) {
+void launch_density_alpha(const DevState<Real>* d, uint32_t n, uint32_t coef_stride, bool warm_v, bool features,
+                          cudaStream_t s) {
     if (!n) return;
-    launch_pdl(density_alpha_kernel<Real>, grid_for(n), kBlock, 0, s, d, n, warm_v && !features, features);
+    launch_pdl(density_alpha_kernel<Real>, grid_for(n), kBlock, 0, s, d, n, warm_v && !features, features, coef_stride);
 }
 template <class Real> void launch_pair_coefficients(const DevState<Real>* d, uint32_t n, cudaStream_t s) {
     if (n) launch_pdl(pair_coefficients_kernel<Real>, grid_for(n), kBlock, 0, s, d, n);
@@ -1180,11 +1205,14 @@ template <class Real> void launch_volumes(const DevState<Real>* d, uint32_t n, c
     if (n) launch_pdl(volumes_kernel<Real>, grid_for(n), kBlock, 0, s, d, n);
 }
 template <class Real>
-void launch_divergence_warm_jacobi(const DevState<Real>* d, uint32_t n, const Real* kw, Vec4<Real>* vout,
+void launch_divergence_warm_jacobi(const DevState<Real>* d, uint32_t n, bool table, const Real* kw, Vec4<Real>* vout,
                                    cudaStream_t s, bool forces) {
     if (!n) return;
-    if (forces) launch_pdl(divergence_warm_jacobi_kernel<Real, true>, grid_for(n), kBlock, 0, s, d, n, kw, vout);
-    else launch_pdl(divergence_warm_jacobi_kernel<Real, false>, grid_for(n), kBlock, 0, s, d, n, kw, vout);
+    with_table(table, [&](auto t) {
+        constexpr bool kT = decltype(t)::value;
+        launch_pdl(forces ? divergence_warm_jacobi_kernel<Real, true, kT> : divergence_warm_jacobi_kernel<Real, false, kT>,
+                   grid_for(n), kBlock, 0, s, d, n, kw, vout);
+    });
 }
 template <class Real>
 void launch_warm_values(const DevState<Real>* d, uint32_t n, int which, bool learned, bool use_pred, double damping,
@@ -1203,19 +1231,24 @@ void launch_gather_training(const DevState<Real>* d, uint32_t n, uint32_t batch,
     if (n && batch) launch_pdl(gather_training_kernel<Real>, grid_for(batch), kBlock, 0, s, d, n, batch, offset, div_ran, x, t);
 }
 template <class Real>
-void launch_divergence_residual(const DevState<Real>* d, uint32_t n, bool init, double eta, int min_it, int max_it,
+void launch_divergence_residual(const DevState<Real>* d, uint32_t n, bool table, bool init, double eta, int min_it, int max_it,
                                 cudaGraphConditionalHandle h, bool use_handle, cudaStream_t s, bool keep) {
     const unsigned g = grid_for(n ? n : 1);
-    auto k = init ? (keep ? divergence_residual_kernel<Real, kInitPass, true> : divergence_residual_kernel<Real, kInitPass, false>)
-                  : (keep ? divergence_residual_kernel<Real, kLoop, true> : divergence_residual_kernel<Real, kLoop, false>);
-    launch_pdl(k, g, kBlock, 0, s, d, n, eta, min_it, max_it, h, use_handle);
+    with_table(table, [&](auto t) {
+        constexpr bool kT = decltype(t)::value;
+        auto k = init ? (keep ? divergence_residual_kernel<Real, kInitPass, true, kT> : divergence_residual_kernel<Real, kInitPass, false, kT>)
+                      : (keep ? divergence_residual_kernel<Real, kLoop, true, kT> : divergence_residual_kernel<Real, kLoop, false, kT>);
+        launch_pdl(k, g, kBlock, 0, s, d, n, eta, min_it, max_it, h, use_handle);
+    });
 }
 template <class Real>
-void launch_divergence_jacobi(const DevState<Real>* d, uint32_t n, cudaGraphConditionalHandle h, bool use_handle,
-                              cudaStream_t s, bool forces) {
+void launch_divergence_jacobi(const DevState<Real>* d, uint32_t n, bool table, cudaGraphConditionalHandle h,
+                              bool use_handle, cudaStream_t s, bool forces) {
     if (!n) return;
-    if (forces) launch_pdl(divergence_jacobi_kernel<Real, true>, grid_for(n), kBlock, 0, s, d, n, h, use_handle);
-    else launch_pdl(divergence_jacobi_kernel<Real, false>, grid_for(n), kBlock, 0, s, d, n, h, use_handle);
+    with_table(table, [&](auto t) {
+        constexpr bool kT = decltype(t)::value;
+        launch_pdl(forces ? divergence_jacobi_kernel<Real, true, kT> : divergence_jacobi_kernel<Real, false, kT>, grid_for(n), kBlock, 0, s, d, n, h, use_handle);
+    });
 }
 template <class Real> void launch_viscosity(const DevState<Real>* d, uint32_t n, bool cfl, cudaStream_t s) {
     if (!n) return;
@@ -1226,56 +1259,59 @@ template <class Real> void launch_update_vel(const DevState<Real>* d, uint32_t n
     if (n) launch_pdl(update_vel_kernel<Real>, grid_for(n), kBlock, 0, s, d, n);
 }
 template <class Real>
-void launch_pressure_warm_jacobi(const DevState<Real>* d, uint32_t n, bool fused_vel, const Real* kw,
+void launch_pressure_warm_jacobi(const DevState<Real>* d, uint32_t n, bool table, bool fused_vel, const Real* kw,
                                  Vec4<Real>* vout, cudaStream_t s, bool forces) {
     if (!n) return;
-    const unsigned g = grid_for(n);
-    if (forces) {
-        if (fused_vel) launch_pdl(pressure_warm_jacobi_kernel<Real, true, true>, g, kBlock, 0, s, d, n, kw, vout);
-        else launch_pdl(pressure_warm_jacobi_kernel<Real, false, true>, g, kBlock, 0, s, d, n, kw, vout);
-    } else {
-        if (fused_vel) launch_pdl(pressure_warm_jacobi_kernel<Real, true, false>, g, kBlock, 0, s, d, n, kw, vout);
-        else launch_pdl(pressure_warm_jacobi_kernel<Real, false, false>, g, kBlock, 0, s, d, n, kw, vout);
-    }
+    with_table(table, [&](auto t) {
+        constexpr bool kT = decltype(t)::value;
+        auto k = forces ? (fused_vel ? pressure_warm_jacobi_kernel<Real, true, true, kT> : pressure_warm_jacobi_kernel<Real, false, true, kT>)
+                        : (fused_vel ? pressure_warm_jacobi_kernel<Real, true, false, kT> : pressure_warm_jacobi_kernel<Real, false, false, kT>);
+        launch_pdl(k, grid_for(n), kBlock, 0, s, d, n, kw, vout);
+    });
 }
 template <class Real>
-void launch_pressure_residual(const DevState<Real>* d, uint32_t n, bool init, double eta, int min_it, int max_it,
-                              cudaGraphConditionalHandle h, bool use_handle, cudaStream_t s, bool keep) {
+void launch_pressure_residual(const DevState<Real>* d, uint32_t n, bool table, bool init, double eta, int min_it, int max_it,
+                                cudaGraphConditionalHandle h, bool use_handle, cudaStream_t s, bool keep) {
     const unsigned g = grid_for(n ? n : 1);
-    auto k = init ? (keep ? pressure_residual_kernel<Real, kInitPass, true> : pressure_residual_kernel<Real, kInitPass, false>)
-                  : (keep ? pressure_residual_kernel<Real, kLoop, true> : pressure_residual_kernel<Real, kLoop, false>);
-    launch_pdl(k, g, kBlock, 0, s, d, n, eta, min_it, max_it, h, use_handle);
+    with_table(table, [&](auto t) {
+        constexpr bool kT = decltype(t)::value;
+        auto k = init ? (keep ? pressure_residual_kernel<Real, kInitPass, true, kT> : pressure_residual_kernel<Real, kInitPass, false, kT>)
+                      : (keep ? pressure_residual_kernel<Real, kLoop, true, kT> : pressure_residual_kernel<Real, kLoop, false, kT>);
+        launch_pdl(k, g, kBlock, 0, s, d, n, eta, min_it, max_it, h, use_handle);
+    });
 }
 template <class Real>
-void launch_warm_dual(const DevState<Real>* d, uint32_t n, int which, bool fused_vel, cudaStream_t s, bool forces) {
+void launch_warm_dual(const DevState<Real>* d, uint32_t n, bool table, int which, bool fused_vel, cudaStream_t s, bool forces) {
     if (!n) return;
-    if (which == 0) {
-        if (forces) launch_pdl(divergence_warm_dual_kernel<Real, true>, grid_for(n), kBlock, 0, s, d, n);
-        else launch_pdl(divergence_warm_dual_kernel<Real, false>, grid_for(n), kBlock, 0, s, d, n);
-    } else if (fused_vel) {
-        if (forces) launch_pdl(pressure_warm_dual_kernel<Real, true, true>, grid_for(n), kBlock, 0, s, d, n);
-        else launch_pdl(pressure_warm_dual_kernel<Real, true, false>, grid_for(n), kBlock, 0, s, d, n);
-    } else {
-        if (forces) launch_pdl(pressure_warm_dual_kernel<Real, false, true>, grid_for(n), kBlock, 0, s, d, n);
-        else launch_pdl(pressure_warm_dual_kernel<Real, false, false>, grid_for(n), kBlock, 0, s, d, n);
-    }
+    with_table(table, [&](auto t) {
+        constexpr bool kT = decltype(t)::value;
+        auto k = which == 0 ? (forces ? divergence_warm_dual_kernel<Real, true, kT> : divergence_warm_dual_kernel<Real, false, kT>)
+                 : forces   ? (fused_vel ? pressure_warm_dual_kernel<Real, true, true, kT> : pressure_warm_dual_kernel<Real, false, true, kT>)
+                            : (fused_vel ? pressure_warm_dual_kernel<Real, true, false, kT> : pressure_warm_dual_kernel<Real, false, false, kT>);
+        launch_pdl(k, grid_for(n), kBlock, 0, s, d, n);
+    });
 }
 template <class Real>
-void launch_residual_dual(const DevState<Real>* d, uint32_t n, int which, double eta, int min_it, int max_it,
+void launch_residual_dual(const DevState<Real>* d, uint32_t n, bool table, int which, double eta, int min_it, int max_it,
                           cudaStream_t s) {
     if (!n) return;
-    if (which == 0) launch_pdl(divergence_residual_dual_kernel<Real>, grid_for(n), kBlock, 0, s, d, n, eta, min_it, max_it);
-    else launch_pdl(pressure_residual_dual_kernel<Real>, grid_for(n), kBlock, 0, s, d, n, eta, min_it, max_it);
+    with_table(table, [&](auto t) {
+        constexpr bool kT = decltype(t)::value;
+        launch_pdl(which == 0 ? divergence_residual_dual_kernel<Real, kT> : pressure_residual_dual_kernel<Real, kT>, grid_for(n),
+                   kBlock, 0, s, d, n, eta, min_it, max_it);
+    });
 }
 template <class Real> void launch_select_candidate(const DevState<Real>* d, uint32_t n, int which, cudaStream_t s) {
     launch_pdl(select_candidate_kernel<Real>, grid_for(n ? n : 1), kBlock, 0, s, d, n, which);
 }
 template <class Real>
-void launch_pressure_jacobi(const DevState<Real>* d, uint32_t n, cudaGraphConditionalHandle h, bool use_handle,
-                            cudaStream_t s, bool forces) {
+void launch_pressure_jacobi(const DevState<Real>* d, uint32_t n, bool table, cudaGraphConditionalHandle h,
+                              bool use_handle, cudaStream_t s, bool forces) {
     if (!n) return;
-    if (forces) launch_pdl(pressure_jacobi_kernel<Real, true>, grid_for(n), kBlock, 0, s, d, n, h, use_handle);
-    else launch_pdl(pressure_jacobi_kernel<Real, false>, grid_for(n), kBlock, 0, s, d, n, h, use_handle);
+    with_table(table, [&](auto t) {
+        constexpr bool kT = decltype(t)::value;
+        launch_pdl(forces ? pressure_jacobi_kernel<Real, true, kT> : pressure_jacobi_kernel<Real, false, kT>, grid_for(n), kBlock, 0, s, d, n, h, use_handle);
+    });
 }
 template <class Real>
 void launch_update_pos(DevState<Real>* d, uint32_t n, cudaStream_t s, const EscapeBox& box, bool end_step) {
@@ -1286,32 +1322,32 @@ template <class Real> void launch_cfl(DevState<Real>* d, uint32_t n_blocks, cons
 }
 
 #define DFSPH_INSTANTIATE_SOLVER(R)                                                                                  \
-    template void launch_density_alpha<R>(const DevState<R>*, uint32_t, bool, bool, cudaStream_t);                  \
+    template void launch_density_alpha<R>(const DevState<R>*, uint32_t, uint32_t, bool, bool, cudaStream_t);                \
     template void launch_pair_coefficients<R>(const DevState<R>*, uint32_t, cudaStream_t);                           \
     template void launch_volumes<R>(const DevState<R>*, uint32_t, cudaStream_t);                                     \
-    template void launch_divergence_warm_jacobi<R>(const DevState<R>*, uint32_t, const R*, Vec4<R>*, cudaStream_t,  \
+    template void launch_divergence_warm_jacobi<R>(const DevState<R>*, uint32_t, bool, const R*, Vec4<R>*, cudaStream_t, \
                                                    bool);                                                            \
-    template void launch_warm_values<R>(const DevState<R>*, uint32_t, int, bool, bool, double, cudaStream_t);       \
-    template void launch_totals<R>(const DevState<R>*, uint32_t, bool, cudaStream_t);                               \
+    template void launch_warm_values<R>(const DevState<R>*, uint32_t, int, bool, bool, double, cudaStream_t);        \
+    template void launch_totals<R>(const DevState<R>*, uint32_t, bool, cudaStream_t);                                \
     template void launch_restore_totals<R>(const DevState<R>*, uint32_t, cudaStream_t);                              \
-    template void launch_gather_training<R>(const DevState<R>*, uint32_t, uint32_t, uint32_t, bool, float*, float*, \
+    template void launch_gather_training<R>(const DevState<R>*, uint32_t, uint32_t, uint32_t, bool, float*, float*,  \
                                             cudaStream_t);                                                           \
-    template void launch_divergence_residual<R>(const DevState<R>*, uint32_t, bool, double, int, int,               \
+    template void launch_divergence_residual<R>(const DevState<R>*, uint32_t, bool, bool, double, int, int,          \
                                                 cudaGraphConditionalHandle, bool, cudaStream_t, bool);               \
-    template void launch_divergence_jacobi<R>(const DevState<R>*, uint32_t, cudaGraphConditionalHandle, bool,       \
+    template void launch_divergence_jacobi<R>(const DevState<R>*, uint32_t, bool, cudaGraphConditionalHandle, bool,  \
                                               cudaStream_t, bool);                                                   \
-    template void launch_viscosity<R>(const DevState<R>*, uint32_t, bool, cudaStream_t);                            \
-    template void launch_update_vel<R>(const DevState<R>*, uint32_t, cudaStream_t);                                 \
-    template void launch_pressure_warm_jacobi<R>(const DevState<R>*, uint32_t, bool, const R*, Vec4<R>*,            \
+    template void launch_viscosity<R>(const DevState<R>*, uint32_t, bool, cudaStream_t);                             \
+    template void launch_update_vel<R>(const DevState<R>*, uint32_t, cudaStream_t);                                  \
+    template void launch_pressure_warm_jacobi<R>(const DevState<R>*, uint32_t, bool, bool, const R*, Vec4<R>*,       \
                                                  cudaStream_t, bool);                                                \
-    template void launch_pressure_residual<R>(const DevState<R>*, uint32_t, bool, double, int, int,                 \
+    template void launch_pressure_residual<R>(const DevState<R>*, uint32_t, bool, bool, double, int, int,            \
                                               cudaGraphConditionalHandle, bool, cudaStream_t, bool);                 \
-    template void launch_warm_dual<R>(const DevState<R>*, uint32_t, int, bool, cudaStream_t, bool);                  \
-    template void launch_residual_dual<R>(const DevState<R>*, uint32_t, int, double, int, int, cudaStream_t);        \
+    template void launch_warm_dual<R>(const DevState<R>*, uint32_t, bool, int, bool, cudaStream_t, bool);            \
+    template void launch_residual_dual<R>(const DevState<R>*, uint32_t, bool, int, double, int, int, cudaStream_t);  \
     template void launch_select_candidate<R>(const DevState<R>*, uint32_t, int, cudaStream_t);                       \
-    template void launch_pressure_jacobi<R>(const DevState<R>*, uint32_t, cudaGraphConditionalHandle, bool,         \
+    template void launch_pressure_jacobi<R>(const DevState<R>*, uint32_t, bool, cudaGraphConditionalHandle, bool,    \
                                             cudaStream_t, bool);                                                     \
-    template void launch_update_pos<R>(DevState<R>*, uint32_t, cudaStream_t, const EscapeBox&, bool);               \
+    template void launch_update_pos<R>(DevState<R>*, uint32_t, cudaStream_t, const EscapeBox&, bool);                \
     template void launch_cfl<R>(DevState<R>*, uint32_t, const DtArgs&, cudaStream_t);
 
 DFSPH_INSTANTIATE_SOLVER(float)

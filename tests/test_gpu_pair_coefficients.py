@@ -110,3 +110,54 @@ def test_passes_without_a_density_pass(n, precision):
         out.append((its, d.field("velocity", np.float64).tobytes(), d.field("kappa", np.float64).tobytes(),
                     d.field("acceleration", np.float64).tobytes()))
     assert out[0] == out[1]
+
+
+FIELDS = ("density", "factor", "velocity", "position", "kappa", "kappa_v", "acceleration", "boundary_force")
+
+
+def _state(d):
+    return [d.field(name, np.float64).tobytes() for name in FIELDS]
+
+
+@pytest.mark.parametrize("learned", [False, True])
+@pytest.mark.parametrize("precision", [32, 64])
+@pytest.mark.parametrize("n", [1, 2, 31, 33, 130, 257, 1025])
+def test_without_the_table(n, precision, learned):
+    """Without the coefficient table the passes evaluate the kernel: the same bits over the list remainders,
+    with forces on a moving boundary and both warm starts; and the table can come and go between steps."""
+    s = _sparse_block(n, seed=n)
+    out = []
+    for tables in ((1, 1, 1, 1), (0, 0, 0, 0), (1, 0, 0, 1)):
+        d = DFSPHCUDA(s, precision=precision)
+        d.set_param("boundary_forces", 1)
+        if learned:
+            d.set_param("train_start", 2)
+            d.set_learned_warm_start(True)
+        got = []
+        for k, table in enumerate(tables):
+            d.set_param("pair_table", table)
+            assert d.get_param("pair_table") == table
+            d.move_boundary_rigid(0, s.boundary.shape[0], None, (2e-4 * k, 0.0, 0.0), (0.2, 0.0, 0.0), None)
+            st = d.step()
+            got += [st.iterations, st.iterations_v, _state(d)]
+        out.append(got)
+    assert out[0] == out[1] == out[2]
+
+
+def test_a_context_that_fills_the_device_takes_no_table():
+    """Lists of 0.3 of the device's memory: with as large a table less than half would stay free."""
+    import torch
+
+    s = _sparse_block(1025, seed=5)
+    row = 65535
+    capacity = int(0.3 * torch.cuda.mem_get_info()[1] / (4 * row))
+    out = []
+    for large in (False, True):
+        d = DFSPHCUDA(s, **(dict(fluid_capacity=capacity, neighbor_capacity=row) if large else {}))
+        assert d.get_param("pair_table") == (0 if large else 1)
+        d.set_param("boundary_forces", 1)
+        for _ in range(2):
+            d.step()
+        out.append(_state(d))
+        d.close()
+    assert out[0] == out[1]
