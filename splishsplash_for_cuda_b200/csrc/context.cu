@@ -277,7 +277,12 @@ public:
     int take_table() {
         coef_ok = false;
         DF_TRY(invalidate_graphs());
-        DF_CUDA(cudaMalloc((void**)&coef, table_bytes()));
+        const cudaError_t e = cudaMalloc((void**)&coef, table_bytes());
+        if (e != cudaSuccess) {
+            coef = nullptr;
+            cudaGetLastError();  // the context works on without it
+        }
+        DF_CUDA(e);
         return DFSPH_OK;
     }
     int drop_table() {
@@ -354,7 +359,10 @@ public:
         use_graphs = s.use_graphs != 0;
         size_t free_bytes = 0, total_bytes = 0;
         DF_CUDA(cudaMemGetInfo(&free_bytes, &total_bytes));
-        if (free_bytes >= table_bytes() + total_bytes / 2) DF_TRY(take_table());
+        if (free_bytes >= table_bytes() + total_bytes / 2) {
+            const int r = take_table();
+            if (r != DFSPH_E_NOMEM) DF_TRY(r);
+        }
         DF_TRY(sync_state());
         reset_dt();
         return DFSPH_OK;

@@ -161,3 +161,26 @@ def test_a_context_that_fills_the_device_takes_no_table():
         out.append(_state(d))
         d.close()
     assert out[0] == out[1]
+
+
+def test_a_refused_table_leaves_the_context_usable():
+    """A table that cannot fit is refused; the steps that follow are those of a context that never asked."""
+    import torch
+
+    from splishsplash_for_cuda_b200 import _capi
+
+    s = _sparse_block(1025, seed=5)
+    row = 65535
+    capacity = int(0.55 * torch.cuda.mem_get_info()[1] / (4 * row))  # lists of 0.55 of the memory, once
+    d = DFSPHCUDA(s, fluid_capacity=capacity, neighbor_capacity=row)
+    small = DFSPHCUDA(s)
+    for x in (d, small):
+        x.set_param("boundary_forces", 1)
+    with pytest.raises(_capi.DfsphError):
+        d.set_param("pair_table", 1)
+    assert d.get_param("pair_table") == 0
+    for x in (d, small):
+        x.step()
+    assert _state(d) == _state(small)
+    d.close()
+    small.close()
