@@ -184,3 +184,27 @@ def test_a_refused_table_leaves_the_context_usable():
     assert _state(d) == _state(small)
     d.close()
     small.close()
+
+
+def test_contexts_give_their_memory_back():
+    """The device's free memory after a context with every optional array is what it was before."""
+    import torch
+
+    s = synthetic_scene(1, counts=(40, 41, 42))
+
+    def use():
+        d = DFSPHCUDA(s)
+        d.set_param("pair_table", 0)
+        d.set_param("boundary_forces", 1)
+        d.set_learned_warm_start(True)
+        d.step()
+        d.set_param("pair_table", 1)
+        d.step()
+        d.body_wrench([0], [10], [[0.0, 0.0, 0.0]])
+        d.close()
+
+    use()  # what the first use of the library keeps (module, graphs)
+    free = torch.cuda.mem_get_info()[0]
+    for _ in range(5):
+        use()
+    assert free - torch.cuda.mem_get_info()[0] < 5 * s.n_fluid  # a leaked array has at least 4 bytes a particle
