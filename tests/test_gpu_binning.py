@@ -96,3 +96,22 @@ def test_fluid_and_boundary_binnings_alternate(n, precision):
         assert d.status() & (_capi.ST_NEIGHBOR_OVERFLOW | _capi.ST_SORT_TIMEOUT | _capi.ST_ESCAPED) == 0
         assert np.array_equal(c, co)
         assert neighbor_sets(c, l) == neighbor_sets(co, lo)
+
+
+def test_lists_read_before_and_after_a_search():
+    """The lists come in groups of the longest one: none before the first search, a far longer one after a
+    part of the fluid has been pressed together."""
+    r, rng = 0.025, np.random.default_rng(3)
+    x = rng.uniform(0.06, 0.94, (1500, 3)).astype(np.float32)
+    walls = box_wall((0, 0, 0), (1.0, 1.0, 1.0), 2 * r).astype(np.float32)
+    s = Scene(config=Configuration(particleRadius=r), fluid=x, boundary=walls)
+    d = DFSPHCUDA(s)
+    c, l = d.neighbors()
+    assert not c.any()
+    for scale in (1.0, 0.5):  # lists of up to 19 and 87, the oracle holds 96
+        s.fluid = (0.5 + scale * (x - 0.5)).astype(np.float32)
+        d.update_fluid(s.fluid)
+        d.neighbors_search()
+        c, l = d.neighbors()
+        co, lo = Oracle(s, 64).neighbors(row=l.shape[1])
+        assert np.array_equal(c, co) and neighbor_sets(c, l) == neighbor_sets(co, lo)
