@@ -1757,7 +1757,7 @@ public:
 
     // The density pass also writes the pair coefficients and m / rho, which the other passes read.
     void density_pass(bool warm_v, bool features_out) {
-        launch_density_alpha<Real>(ds, n, coef ? stride : 0u, warm_v, features_out, stream);
+        launch_density_alpha<Real>(ds, n, coef != nullptr, warm_v, features_out, stream);
         coef_ok = true;
     }
     // Both of these for a pass that no density pass at these positions precedes.

@@ -123,11 +123,9 @@ void launch_scatter_by_id(const uint32_t* id, uint32_t n, const Real* src, int c
 
 // ---- launch wrappers (solver.cu) ------------------------------------------------------------------
 // table: the coefficient table exists (coef not null); without it the passes form the coefficients.
-// coef_stride: nbr_stride, or 0 without a table (coef then holds one group per particle, not read).
 // warm_v: scale kappa_v into the reference warm start; features: write the MLP inputs instead.
 template <class Real>
-void launch_density_alpha(const DevState<Real>* d, uint32_t n, uint32_t coef_stride, bool warm_v, bool features,
-                          cudaStream_t s);
+void launch_density_alpha(const DevState<Real>* d, uint32_t n, bool table, bool warm_v, bool features, cudaStream_t s);
 // What the density pass leaves for the other passes, where none at these positions precedes them: the pair
 // coefficients and m / rho, or m / rho alone.
 template <class Real> void launch_pair_coefficients(const DevState<Real>* d, uint32_t n, cudaStream_t s);

@@ -395,11 +395,10 @@ __device__ __forceinline__ void jacobi_sum2(const DevState<Real>* __restrict__ d
 }
 
 // Visits the `entries` slots of the groups from idx on two at a time (load(u, j), then f = use(u)) and
-// writes their pair coefficients, 0 for the fill-up slots.
-template <class Real, class Load, class Use>
+// writes their pair coefficients, 0 for the fill-up slots (without a table one group over the other).
+template <bool kTable, class Real, class Load, class Use>
 __device__ __forceinline__ void visit_coefficients(const uint4* __restrict__ idx, Vec4<Real>* __restrict__ coef,
-                                                   uint32_t stride, uint32_t coef_stride, uint32_t entries, Load&& load,
-                                                   Use&& use) {
+                                                   uint32_t stride, uint32_t entries, Load&& load, Use&& use) {
     if (!entries) return;
     uint4 j = ld_group(idx);
     for (uint32_t k = 0; k < entries; k += 4) {
@@ -417,7 +416,7 @@ __device__ __forceinline__ void visit_coefficients(const uint4* __restrict__ idx
         if (k + 2 < entries) f.z = use(0);
         if (k + 3 < entries) f.w = use(1);
         *coef = f;
-        coef += coef_stride;
+        if constexpr (kTable) coef += stride;
         j = jn;
     }
 }
@@ -431,11 +430,12 @@ __device__ __forceinline__ void visit_coefficients(const uint4* __restrict__ idx
 // and four -> three -> two: 180 -> 174 -> 152 -> 100 us at 250 k particles, 588 -> 545 -> 475 -> 328 us at
 // 1 M, 57 -> 52 -> 49 -> 28 us at 27 k. The FP32 build spills 8 bytes at four.
 template <class Real> constexpr int kDensityMinBlocks = std::is_same<Real, double>::value ? 2 : kGatherMinBlocks;
-// Without a coefficient table coef_stride is 0, and a particle's groups go one over the other into a spare array:
-// the same machine code either way, because the compiler contracts the FP32 sums of alpha as it likes.
-template <class Real>
+// Without a coefficient table a particle's coefficients go to a spare array all the same: the compiler contracts
+// the FP32 sums of alpha as it likes, and differently when the coefficients are not formed. With the stores the
+// two instantiations give the same bits; a step passed at run time cost 2 % at 1 M particles.
+template <class Real, bool kTable>
 __global__ void __launch_bounds__(kBlock, kDensityMinBlocks<Real>) density_alpha_kernel(
-    const DevState<Real>* __restrict__ ds, uint32_t n, bool warm_v, bool features, uint32_t coef_stride) {
+    const DevState<Real>* __restrict__ ds, uint32_t n, bool warm_v, bool features) {
     DFSPH_PDL_ENTER;
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
@@ -480,8 +480,8 @@ __global__ void __launch_bounds__(kBlock, kDensityMinBlocks<Real>) density_alpha
     };
     {
         Vec4<Real> xj[2], vj[2];
-        visit_coefficients<Real>(
-            ds->nbr + i, ds->coef + i, stride, coef_stride, nf,
+        visit_coefficients<kTable, Real>(
+            ds->nbr + i, ds->coef + i, stride, nf,
             [&](int u, uint32_t j) {
                 xj[u] = ld4<Real>(pos + j);
                 vj[u] = ld4<Real>(vel + j);
@@ -502,9 +502,9 @@ __global__ void __launch_bounds__(kBlock, kDensityMinBlocks<Real>) density_alpha
     if (nb) {
         const bool moving = p.boundary_moving != 0;
         BNbr<Real> b[2];
-        const size_t g = slot_groups(nf);
-        visit_coefficients<Real>(
-            ds->nbr + g * stride + i, ds->coef + g * coef_stride + i, stride, coef_stride, nb,
+        const size_t at = (size_t)slot_groups(nf) * stride + i;
+        visit_coefficients<kTable, Real>(
+            ds->nbr + at, ds->coef + (kTable ? at : i), stride, nb,
             [&](int u, uint32_t j) { load_bnbr(b[u], ds->bpos, ds->bvel, j, moving); },
             [&](int u) {
                 const Real rx = xi.x - b[u].x.x, ry = xi.y - b[u].x.y, rz = xi.z - b[u].x.z;
@@ -551,8 +551,8 @@ __global__ void __launch_bounds__(kBlock, kGatherMinBlocks) pair_coefficients_ke
     const uint32_t nf = fluid_count(c), nb = boundary_count(c);
     Vec4<Real> xj[2];
     auto rows = [&](const Vec4<Real>* __restrict__ src, size_t at, uint32_t entries) {
-        visit_coefficients<Real>(
-            ds->nbr + at, ds->coef + at, stride, stride, entries, [&](int u, uint32_t j) { xj[u] = ld4<Real>(src + j); },
+        visit_coefficients<true, Real>(
+            ds->nbr + at, ds->coef + at, stride, entries, [&](int u, uint32_t j) { xj[u] = ld4<Real>(src + j); },
             [&](int u) { return K.pair_factor(xi.x - xj[u].x, xi.y - xj[u].y, xi.z - xj[u].z); });
     };
     rows(ds->pos, i, nf);
@@ -1193,10 +1193,11 @@ template <class F> static void with_table(bool table, F&& f) {
 }
 
 template <class Real>
-void launch_density_alpha(const DevState<Real>* d, uint32_t n, uint32_t coef_stride, bool warm_v, bool features,
-                          cudaStream_t s) {
+void launch_density_alpha(const DevState<Real>* d, uint32_t n, bool table, bool warm_v, bool features, cudaStream_t s) {
     if (!n) return;
-    launch_pdl(density_alpha_kernel<Real>, grid_for(n), kBlock, 0, s, d, n, warm_v && !features, features, coef_stride);
+    with_table(table, [&](auto t) {
+        launch_pdl(density_alpha_kernel<Real, decltype(t)::value>, grid_for(n), kBlock, 0, s, d, n, warm_v && !features, features);
+    });
 }
 template <class Real> void launch_pair_coefficients(const DevState<Real>* d, uint32_t n, cudaStream_t s) {
     if (n) launch_pdl(pair_coefficients_kernel<Real>, grid_for(n), kBlock, 0, s, d, n);
@@ -1322,7 +1323,7 @@ template <class Real> void launch_cfl(DevState<Real>* d, uint32_t n_blocks, cons
 }
 
 #define DFSPH_INSTANTIATE_SOLVER(R)                                                                                  \
-    template void launch_density_alpha<R>(const DevState<R>*, uint32_t, uint32_t, bool, bool, cudaStream_t);                \
+    template void launch_density_alpha<R>(const DevState<R>*, uint32_t, bool, bool, bool, cudaStream_t);                    \
     template void launch_pair_coefficients<R>(const DevState<R>*, uint32_t, cudaStream_t);                           \
     template void launch_volumes<R>(const DevState<R>*, uint32_t, cudaStream_t);                                     \
     template void launch_divergence_warm_jacobi<R>(const DevState<R>*, uint32_t, bool, const R*, Vec4<R>*, cudaStream_t, \
