@@ -297,6 +297,7 @@ public:
         DF_TRY(invalidate_graphs());
         return sync_state();
     }
+    static constexpr size_t kSmallTable = 64u << 20;
     size_t table_bytes() const { return (size_t)group_capacity(cap) * stride * sizeof(Vec4<Real>); }
 
     int init(const dfsph_scene& s) {
@@ -371,9 +372,10 @@ public:
         DF_CUDA(cudaEventCreateWithFlags(&ev_vel_free, cudaEventDisableTiming));
         time_step = s.time_step;
         use_graphs = s.use_graphs != 0;
+        // (a small table without the look at the free memory, which takes 70 us)
         size_t free_bytes = 0, total_bytes = 0;
-        DF_CUDA(cudaMemGetInfo(&free_bytes, &total_bytes));
-        if (free_bytes >= table_bytes() + total_bytes / 2) {
+        if (table_bytes() > kSmallTable) DF_CUDA(cudaMemGetInfo(&free_bytes, &total_bytes));
+        if (table_bytes() <= kSmallTable || free_bytes >= table_bytes() + total_bytes / 2) {
             const int r = take_table();
             if (r != DFSPH_E_NOMEM) DF_TRY(r);
         }
