@@ -208,8 +208,8 @@ int dfsph_upload_fluid(dfsph_ctx* ctx, const float* xyz, const float* vxyz, cons
  * DFSPH_c_arrays_structure.cpp:1120; the reference has no fluid upload between steps). vxyz null sets the velocities
  * to zero. The copies are asynchronous: from page-locked host memory the buffers must stay unchanged
  * until the next call that waits (dfsph_step with stats, a read, dfsph_synchronize). The velocities
- * travel on a second stream and are applied inside the next step's binning, after its sort, or by
- * whichever other call on the context comes first, so every call sees the new state. */
+ * travel on a second stream and are applied by the next step or neighbour search after it has built its
+ * lists, or by whichever other call on the context comes first, so every call sees the new state. */
 int dfsph_update_fluid(dfsph_ctx* ctx, const float* xyz, const float* vxyz);
 
 /* Copies a field to host memory. n_elems is the capacity of out in elements of dtype; the call

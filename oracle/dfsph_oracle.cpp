@@ -108,8 +108,8 @@ template <class Real> struct Cubic {
 };
 
 // Density terms m_j W_ij of the FP32 instance, evaluated in FP64 from the FP32 distance components
-// and summed in FP64, as the device's density_term (dfsph_common.cuh). The FP64 instance evaluates
-// the terms with its kernel.
+// and summed in FP64. The device's density_term (dfsph_common.cuh) forms the same terms with FMAs and a Newton
+// root, so the two agree to FP64 rounding. The FP64 instance evaluates the terms with its kernel.
 struct DensityTerms {
     double ih2 = 0, k = 0;
     void set(double H) {

@@ -275,8 +275,8 @@ template <class Real> struct Cubic {
 // sums rho - rho0 in FP64 from these terms.
 // q = sqrt(q2) comes from the FP32 reciprocal square root and two Newton steps (Heron's method in its
 // division-free form, relative error 2^-22 -> 2^-44 -> rounding) instead of the correctly rounded FP64
-// square root: density pass 240 -> 205 us at 1 M particles, the stored densities of 27 k to 150 k
-// particles bit for bit the same. The self term (r = 0) is m k.
+// square root: density pass 219 -> 212 us at 1 M particles, 412 -> 399 us at 2 M, the stored densities of 27 k
+// and 250 k particles bit for bit the same. The self term (r = 0) is m k.
 __device__ __forceinline__ double density_term(const Cubic<float>& K, float rx, float ry, float rz, float m) {
     const double dx = rx, dy = ry, dz = rz;
     const double q2 = fma(dz, dz, fma(dy, dy, dx * dx)) * K.ih2_d;

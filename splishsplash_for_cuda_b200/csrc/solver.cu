@@ -40,8 +40,8 @@ __device__ __forceinline__ uint32_t boundary_count(uint32_t c) { return c >> 16;
 // Visits the block partials b = threadIdx.x, threadIdx.x + kBlock, ... < count in that order, eight loads in
 // flight: the last block walks them alone while the chip waits, and one at a time each costs a trip to L2.
 // Relaxed loads at GPU scope: other blocks wrote the values. One at a time -> eight: step 8.25 -> 8.19 ms
-// at 4 M particles (15,625 partials a pass), 2.21 -> 2.20 at 1 M, unchanged at 250 k and below; four at a
-// time measure the same.
+// at 4 M particles (15,625 partials a pass), no difference beyond the runs' at 1 M and below; four at a time
+// measure the same.
 constexpr int kPartialBatch = 8;
 __device__ __forceinline__ double ld_partial(const double* p) {
     double v;
@@ -669,8 +669,8 @@ __global__ void __launch_bounds__(kBlock, kGatherMinBlocks) divergence_jacobi_ke
 
 // XSPH viscosity + gravity: a_i = g - sum (inv_h * nu * m_j / rho_j) (v_i - v_j) W_ij over fluid
 // neighbours. With kCfl the block maximum of |v + a h|^2 is stored for the CFL time step.
-// The viscosity pass gathers position, velocity and density: at four neighbours per batch it spills
-// at the 64-register cap; two per batch runs without spills, 14 % faster at 1 M particles.
+// The pass gathers position, velocity and m / rho. Two neighbours per batch: at four it spilled at the
+// 64-register cap (when it gathered the density; two were 14 % faster at 1 M particles).
 template <class Real, bool kCfl>
 __global__ void __launch_bounds__(kBlock, kGatherMinBlocks) viscosity_kernel(const DevState<Real>* __restrict__ ds, uint32_t n) {
     DFSPH_PDL_ENTER;
