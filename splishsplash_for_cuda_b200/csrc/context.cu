@@ -279,6 +279,7 @@ public:
     // it, 598 B and 2.37 ms without (602 B and 2.57 ms before there was one); 4 M: 7.99 and 8.85 ms.
     int take_table() {
         coef_ok = false;
+        DF_CUDA(cudaStreamSynchronize(stream));  // a loop graph may still run
         DF_TRY(invalidate_graphs());
         const cudaError_t e = cudaMalloc((void**)&coef, table_bytes());
         if (e != cudaSuccess) {
